@@ -10,6 +10,7 @@
 // reproduces it bit for bit.  Compiled without FMA contraction so the float
 // quantisation step rounds like the host build.
 #include "lbvh_build.h"
+#include "lbvh_pack.h"
 
 #include <cuda_runtime.h>
 #include <cfloat>
@@ -781,7 +782,8 @@ uint32_t lbvhMaxLeafDepth(uint32_t n, const int32_t* children, void* scratch, cu
 }
 
 // Leaves below every internal node, bottom up: the second arrival at a node
-// adds its children's counts.
+// adds its children's counts.  (A node of a malformed hierarchy may see more
+// arrivals; those end there, so that none goes round a cycle.)
 __global__ void leafCountKernel(int n, const int32_t* children, const int32_t* parentOfNode,
                                 const int32_t* parentOfLeaf, uint32_t* arrivals, uint32_t* count) {
     const int leaf = blockIdx.x * blockDim.x + threadIdx.x;
@@ -789,7 +791,7 @@ __global__ void leafCountKernel(int n, const int32_t* children, const int32_t* p
     int node = parentOfLeaf[leaf];
     while (node >= 0 && node < n - 1) {
         __threadfence();
-        if (atomicAdd(&arrivals[node], 1u) == 0u) return;
+        if (atomicAdd(&arrivals[node], 1u) != 1u) return;
         __threadfence();
         uint32_t c = 0;
         for (int k = 0; k < 2; ++k) {
@@ -801,48 +803,41 @@ __global__ void leafCountKernel(int n, const int32_t* children, const int32_t* p
     }
 }
 
-// One thread per node: its place in depth-first order (a node's first child
-// follows it, the second child follows the first's subtree) and the place of
-// its first leaf among the leaves, summed on the way up to the root.  A ray
-// that goes on to a node's first child finds it in the next 64 bytes, and a
-// subtree's nodes and triangles are contiguous: terrain scene of 3.4 M
+// One thread per node: writes it at its place in depth-first order (placeNode).
+// A ray that goes on to a node's first child finds it in the next 64 bytes,
+// and a subtree's nodes and triangles are contiguous: terrain scene of 3.4 M
 // triangles, traversal 8.70 -> 8.52 ms per 4-spp frame.
 __global__ void packTraversalKernel(const BvhNode* nodes, const int32_t* children, const int32_t* parentOfNode,
-                                    const uint32_t* count, const BvhTri* tris, uint32_t n, TravNode* outNodes,
-                                    BvhTri* outTris, uint32_t* errorFlag) {
+                                    const int32_t* parentOfLeaf, const uint32_t* count, const BvhTri* tris, uint32_t n,
+                                    TravNode* outNodes, BvhTri* outTris, uint32_t* errorFlag) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i + 1 >= n) return;
-    const int last = static_cast<int>(n) - 1;
-    uint32_t place = 0, firstLeaf = 0, steps = 0;
-    int node = static_cast<int>(i);
-    for (int up = parentOfNode[node]; up >= 0 && up < last && steps < n; up = parentOfNode[node], ++steps) {
-        const int left = children[2 * up];
-        place += 1;
-        if (left != node) {
-            const uint32_t leaves = left >= 0 && left < last ? count[left] : 1u;
-            place += leaves - 1;
-            firstLeaf += leaves;
-        }
-        node = up;
-    }
     const BvhNode nd = nodes[i];
     const int c0 = __float_as_int(nd.lo0.w), c1 = __float_as_int(nd.lo1.w);
-    const uint32_t leaves0 = c0 >= 0 && c0 < last ? count[c0] : 1u;
-    const uint32_t leaf1 = firstLeaf + leaves0;
-    const uint32_t node0 = place + 1, node1 = place + leaves0;
-    const bool ok = c0 < last && c1 < last && ~c0 <= last && ~c1 <= last && node == 0 &&
-                    place < n - 1 && leaf1 < n && (c0 < 0 || node0 < n - 1) && (c1 < 0 || node1 < n - 1);
-    if (!ok) { atomicOr(errorFlag, 1u); return; }
+    PackedNode pl;
+    if (c0 != children[2 * i] || c1 != children[2 * i + 1] ||
+        !placeNode(children, parentOfNode, parentOfLeaf, count, n, i, &pl)) {
+        atomicOr(errorFlag, 1u);
+        return;
+    }
     TravNode t;
     t.x = make_float4(nd.lo0.x, nd.lo1.x, nd.hi0.x, nd.hi1.x);
     t.y = make_float4(nd.lo0.y, nd.lo1.y, nd.hi0.y, nd.hi1.y);
     t.z = make_float4(nd.lo0.z, nd.lo1.z, nd.hi0.z, nd.hi1.z);
-    t.child0 = c0 >= 0 ? static_cast<int>(node0) : ~static_cast<int>(firstLeaf);
-    t.child1 = c1 >= 0 ? static_cast<int>(node1) : ~static_cast<int>(leaf1);
+    t.child0 = pl.child0;
+    t.child1 = pl.child1;
     t.pad[0] = t.pad[1] = 0;
-    outNodes[place] = t;
-    if (c0 < 0) outTris[firstLeaf] = tris[~c0];
-    if (c1 < 0) outTris[leaf1] = tris[~c1];
+    outNodes[pl.place] = t;
+    if (c0 < 0) outTris[pl.firstLeaf] = tris[~c0];
+    if (c1 < 0) outTris[pl.leaf1] = tris[~c1];
+}
+
+// A hierarchy that is not one tree may pack into references that never end:
+// its root then leads to leaf 0 alone.
+__global__ void closePackedKernel(const uint32_t* errorFlag, TravNode* outNodes) {
+    if (!(*errorFlag & 1u)) return;
+    outNodes[0].child0 = ~0;
+    outNodes[0].child1 = ~0;
 }
 
 void lbvhPackTraversal(const LbvhOutput &built, uint32_t n, void* scratch, TravNode* outNodes, BvhTri* outTris,
@@ -862,7 +857,7 @@ void lbvhPackTraversal(const LbvhOutput &built, uint32_t n, void* scratch, TravN
     ck(cudaMemsetAsync(count, 0, size_t(n) * 4, stream), "leaf counts");
     ck(cudaMemsetAsync(parentOfLeaf, 0xFF, size_t(n) * 4, stream), "leaf parents");
     ck(cudaMemsetAsync(parentOfNode, 0xFF, size_t(n) * 4, stream), "node parents");
-    // a slot that a malformed hierarchy leaves unwritten: no box, references to leaf 0, no hit
+    // a slot that a malformed hierarchy leaves unwritten: references to leaf 0, a triangle that nothing hits
     ck(cudaMemsetAsync(outNodes, 0xFF, size_t(n - 1) * sizeof(TravNode), stream), "traversal nodes");
     ck(cudaMemsetAsync(outTris, 0xFF, size_t(n) * sizeof(BvhTri), stream), "traversal triangles");
     const uint32_t tb = 256;
@@ -870,8 +865,9 @@ void lbvhPackTraversal(const LbvhOutput &built, uint32_t n, void* scratch, TravN
                                                              parentOfLeaf);
     leafCountKernel<<<(n + tb - 1) / tb, tb, 0, stream>>>(static_cast<int>(n), built.children, parentOfNode,
                                                           parentOfLeaf, arrivals, count);
-    packTraversalKernel<<<(n - 1 + tb - 1) / tb, tb, 0, stream>>>(built.nodes, built.children, parentOfNode, count,
-                                                                  built.tris, n, outNodes, outTris, errorFlag);
+    packTraversalKernel<<<(n - 1 + tb - 1) / tb, tb, 0, stream>>>(built.nodes, built.children, parentOfNode, parentOfLeaf,
+                                                                  count, built.tris, n, outNodes, outTris, errorFlag);
+    closePackedKernel<<<1, 1, 0, stream>>>(errorFlag, outNodes);
     ck(cudaGetLastError(), "pack traversal nodes");
 }
 

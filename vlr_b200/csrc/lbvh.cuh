@@ -57,13 +57,14 @@ struct BvhTri {
     float4 v2;   // xyz, w unused
 };
 
-// Every child reference in `nodes` is in range (the packing kernel replaces
-// one that is not and sets errorFlag's bit 0), so traversal does not check.
+// The references in `nodes` are in range and every descent from the root ends:
+// packing checks that they form one tree, else sets errorFlag's bit 0 and lets
+// the root lead to leaf 0 alone.  So traversal does not check.
 struct Bvh {
     const TravNode* nodes;
     const BvhTri* tris;
     uint32_t numTris;
-    uint32_t* errorFlag;   // bit 0: out-of-range node reference met; bit 1: traversal stack overflow
+    uint32_t* errorFlag;   // bit 0: the hierarchy is not one tree; bit 1: traversal stack overflow
 };
 
 struct Hit {

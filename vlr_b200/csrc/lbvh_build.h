@@ -46,9 +46,9 @@ uint32_t lbvhBuildTraversable(const float* verts, uint32_t n, uint32_t rounds, v
                               uint32_t* restructuredDev, cudaStream_t stream);
 
 // The arrays the traversal walks, from the built ones: nodes and triangles
-// in depth-first order, child references checked (a hierarchy that is not a
-// tree over its n leaves sets bit 0 of *errorFlag and keeps every reference
-// in range).  scratch: lbvhTraversableScratchBytes(n).
+// in depth-first order, child references checked (a hierarchy that is not one
+// tree over its n leaves sets bit 0 of *errorFlag, and its root then leads to
+// leaf 0 alone).  scratch: lbvhTraversableScratchBytes(n).
 void lbvhPackTraversal(const LbvhOutput &built, uint32_t n, void* scratch, TravNode* outNodes, BvhTri* outTris,
                        uint32_t* errorFlag, cudaStream_t stream);
 
