@@ -182,3 +182,38 @@ def test_persistent_batch_keeps_guided_items_and_orders_by_work():
     batch.close()
     for c in (small, plain, guided):
         c.close()
+
+
+def test_batch_graph_shares_the_gpu():
+    """A graph of small scenes takes no longer than the same renders issued on
+    a stream of their own each (these overlap too; the best of several rounds
+    of either, a fifth for scatter)."""
+    import torch
+    from vlr_b200 import vlr as VV
+    sizes = [(64, 8), (128, 8), (256, 8), (320, 8)]
+    ctxs = [_ctx(w, w) for w, _ in sizes]
+    for c, _, _ in ctxs:
+        c.setOptions(max_paths_in_flight=1 << 20)
+    streams = [torch.cuda.Stream() for _ in ctxs]
+    batch = VV.RenderBatch([(c, cam, spp, True) for (c, cam, _), (_, spp) in zip(ctxs, sizes)])
+
+    def apart():
+        for (c, cam, _), (_, spp), s in zip(ctxs, sizes, streams):
+            c.render_samples(cam, True, spp, stream=s.cuda_stream)
+
+    def best(f):
+        import time
+        t = []
+        for _ in range(12):
+            torch.cuda.synchronize()
+            t0 = time.perf_counter()
+            f()
+            torch.cuda.synchronize()
+            t.append(time.perf_counter() - t0)
+        return min(t)
+
+    t_apart, t_graph = best(apart), best(batch.launch)
+    batch.close()
+    for c, _, _ in ctxs:
+        c.close()
+    assert t_graph < 1.2 * t_apart, (t_graph, t_apart)

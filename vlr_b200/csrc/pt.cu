@@ -43,13 +43,29 @@ namespace {
 // before it touches memory, so the end of one implies the end of all before
 // it.  Measured on frames of many short launches: 256 x 256, 1 spp 409 -> 400
 // us; small terrain 637 x 359, 4 spp 1.43 -> 1.39 ms; the large ones the same.
+//
+// Not while capturing: in a graph the programmatic edges keep side-by-side
+// branches from sharing the GPU.  Graph of Cornell boxes of 64, 128, 256 and 320
+// pixels a side, 8 spp each: 1.74 ms with them, 1.00 without; twelve of 128, 2
+// spp: 2.47 and 0.89.  (The same renders on streams of their own: 1.21 and 1.13;
+// 1.21 and 1.21.)
 __device__ __forceinline__ void startDependent() {
     cudaTriggerProgrammaticLaunchCompletion();
     cudaGridDependencySynchronize();
 }
 
+struct Chain {
+    cudaStream_t stream;
+    bool programmatic;
+    explicit Chain(cudaStream_t s) : stream(s), programmatic(true) {
+        if (s == nullptr) return;   // the legacy stream cannot be captured
+        cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+        programmatic = cudaStreamIsCapturing(s, &status) == cudaSuccess && status == cudaStreamCaptureStatusNone;
+    }
+};
+
 template <class... Params, class... Args>
-inline void launchChained(void (*kernel)(Params...), uint32_t grid, uint32_t block, cudaStream_t stream,
+inline void launchChained(void (*kernel)(Params...), uint32_t grid, uint32_t block, const Chain &chain,
                           Args &&...args) {
     cudaLaunchAttribute attr{};
     attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -57,9 +73,9 @@ inline void launchChained(void (*kernel)(Params...), uint32_t grid, uint32_t blo
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(block);
-    cfg.stream = stream;
+    cfg.stream = chain.stream;
     cfg.attrs = &attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = chain.programmatic ? 1 : 0;
     const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
     if (e != cudaSuccess) throw std::runtime_error(std::string("pt launch: ") + cudaGetErrorString(e));
 }
@@ -749,6 +765,7 @@ void ptRenderLaunch(const SceneGPU &scene, const PathBuffers &pb, const Film &fi
                                                     (256 / kRayThreads),
                                                 (fp.numPaths + kRayThreads - 1) / kRayThreads);
     const size_t pMain = sizeof(SceneGPU) + sizeof(PathBuffers) + sizeof(FrameParams);
+    const Chain chain(stream);
     ck(cudaMemsetAsync(pb.counters, 0, size_t(kMaxBounces + 1) * kCountersPerBounce * 4, stream), "counters");
     const bool guiding = gfp && (gfp->sample || gfp->record);
     if (guiding && gfp->record) {
@@ -759,8 +776,8 @@ void ptRenderLaunch(const SceneGPU &scene, const PathBuffers &pb, const Film &fi
     for (uint32_t b = 0; b < fp.maxPathLength; ++b) {
         fp.bounce = b;
         T.begin(kStageTrace, stream, pMain);
-        if (b == 0) launchChained(cameraTraceKernel, rayGrid, kRayThreads, stream, scene, pb, fp);
-        else launchChained(traceShadowKernel, rayGrid, kRayThreads, stream, scene, pb, fp);
+        if (b == 0) launchChained(cameraTraceKernel, rayGrid, kRayThreads, chain, scene, pb, fp);
+        else launchChained(traceShadowKernel, rayGrid, kRayThreads, chain, scene, pb, fp);
         T.end(stream);
         if (guiding && gfp->sample && b < gfp->recBounces) {
             GuidedHitSrc src{ scene, pb, fp, gfp->net };
@@ -780,10 +797,10 @@ void ptRenderLaunch(const SceneGPU &scene, const PathBuffers &pb, const Film &fi
         // its records; later bounces only add to the path's contribution,
         // which the plain variant (fewer registers) does the same way
         const bool guideShade = guiding && (b < gfp->recBounces || (gfp->record && b == gfp->recBounces));
-        if (guideShade && maps) launchChained(shadeKernel<true, true>, grid, 256, stream, scene, pb, fp, *gfp);
-        else if (guideShade) launchChained(shadeKernel<true, false>, grid, 256, stream, scene, pb, fp, *gfp);
-        else if (maps) launchChained(shadeKernel<false, true>, grid, 256, stream, scene, pb, fp, GuideFrame{});
-        else launchChained(shadeKernel<false, false>, grid, 256, stream, scene, pb, fp, GuideFrame{});
+        if (guideShade && maps) launchChained(shadeKernel<true, true>, grid, 256, chain, scene, pb, fp, *gfp);
+        else if (guideShade) launchChained(shadeKernel<true, false>, grid, 256, chain, scene, pb, fp, *gfp);
+        else if (maps) launchChained(shadeKernel<false, true>, grid, 256, chain, scene, pb, fp, GuideFrame{});
+        else launchChained(shadeKernel<false, false>, grid, 256, chain, scene, pb, fp, GuideFrame{});
         T.end(stream);
     }
     if (guiding && gfp->record) {
@@ -795,10 +812,10 @@ void ptRenderLaunch(const SceneGPU &scene, const PathBuffers &pb, const Film &fi
                                     sizeof(FilmResolve));
     const uint32_t pixels = fp.width * fp.height;
     launchChained(filmResolveKernel, std::min<uint32_t>((pixels + kFilmThreads - 1) / kFilmThreads, numSMs * 24u),
-                  kFilmThreads, stream, pb, film, fp, filmConst(), resolve);
+                  kFilmThreads, chain, pb, film, fp, filmConst(), resolve);
     T.end(stream);
     T.begin(kStageFilm, stream, sizeof(PathBuffers) + 16 + sizeof(FilmResolve));
-    launchChained(statsKernel, 1, 32, stream, pb, fp.maxPathLength, film.frames, resolve);
+    launchChained(statsKernel, 1, 32, chain, pb, fp.maxPathLength, film.frames, resolve);
     T.end(stream);
     ck(cudaGetLastError(), "launch");
     T.collect();
