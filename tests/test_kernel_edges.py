@@ -105,6 +105,79 @@ def test_film_pass_of_a_shrunk_preview_leaves_the_rest_empty():
     ctx.close()
 
 
+def _glowing_box(W, H, spp):
+    """A context inside a box that only emits, seen through a field of view so
+    narrow that all camera rays weigh the same: every sample adds one value to
+    each quarter of its pixel's strata."""
+    from vlr_b200 import vlr as VV
+    ctx = VV.Context()
+    ctx.bindOutputBuffer(W, H)
+    mat = ctx.createSurfaceMaterial("DiffuseEmitter")
+    mat.set("emittance", VV.rgb(1.0, 1.0, 1.0))
+    node = ctx.createTriangleMeshSurfaceNode("wall")
+    corners = [(-1, -1), (1, -1), (1, 1), (-1, 1)]
+    verts = np.array([[x, y, z, 0, 0, -z, 1, 0, 0, 0, 0] for z in (-1, 1) for x, y in corners], np.float32)
+    node.set_vertices(verts)
+    node.add_material_group(np.array([0, 1, 2, 0, 2, 3, 4, 6, 5, 4, 7, 6], np.uint32), mat)
+    scene = ctx.createScene()
+    scene.add_child(node)
+    cam = ctx.createCamera("Perspective")
+    cam.set_point("position", (0.0, 0.0, 0.0))
+    for k, v in (("aspect", 1.0), ("sensitivity", 1.0), ("fovy", 1e-3), ("lens radius", 0.0), ("op distance", 1.0)):
+        cam.set(k, v)
+    ctx.setScene(scene)
+    ctx.setOptions(max_path_length=2, max_paths_in_flight=max(W * H * spp, 1))
+    return ctx, cam, (scene, node, mat)
+
+
+def _quarters(film, frames):
+    H, W = film.shape[:2]
+    return film.reshape(H, W, 4, 4).sum(axis=3) * (W * H / frames)
+
+
+@pytest.fixture(scope="module")
+def quarter_means():
+    ctx, cam, keep = _glowing_box(256, 256, 16)
+    ctx.render_samples(cam, True, 16)
+    means = _quarters(ctx.read_film(), 16).mean(axis=(0, 1))
+    ctx.close()
+    return means
+
+
+@pytest.mark.parametrize("size,spp", [((1, 1), 1), ((1, 1), 64), ((1, 1), 257), ((7, 3), 2), ((7, 3), 3), ((7, 3), 5),
+                                      ((7, 3), 9), ((33, 17), 16), ((33, 17), 31), ((64, 64), 33), ((129, 65), 64),
+                                      ((320, 200), 12), ((512, 320), 7)])
+def test_film_pass_counts_every_sample_once(quarter_means, size, spp):
+    """However many threads share a pixel, each sample is in its pixel's sums
+    once.  A quarter's sum over n samples is n times a mean over 117.5 nm plus
+    noise: the emission varies by less than a half within a quarter, so its
+    standard error is below 0.5 / sqrt(12 n); six of them, below half a sample for
+    n up to 12, and beyond that over all pixels a loss of one sample in each would
+    stand out by far more."""
+    (W, H), n = size, spp
+    ctx, cam, keep = _glowing_box(W, H, spp)
+    for first, frames in ((True, n), (False, 2 * n)):
+        ctx.render_samples(cam, first, n)
+        rel = _quarters(ctx.read_film(), frames) / quarter_means - 1
+        assert np.all(np.abs(rel) < 6 * 0.5 / np.sqrt(12 * frames)), np.abs(rel).max()
+        assert np.all(np.abs(rel.mean(axis=(0, 1))) < 6 * 0.5 / np.sqrt(12 * frames * W * H) + 2e-3)
+    ctx.close()
+
+
+def test_film_pass_of_few_pixels_splits_their_samples():
+    """64 x 64 pixels of 512 samples are 67 MB of contributions, 10 us of HBM; one
+    thread a pixel took 630."""
+    ctx, cam, keep = _render_context(64, 64, max_paths_in_flight=64 * 64 * 512)
+    ctx.set_profiling(True)
+    ms = []
+    for _ in range(4):
+        ctx.kernel_times(reset=True)
+        ctx.render_samples(cam, True, 512)
+        ms.append(ctx.kernel_times()[0]["film"]["ms"])
+    ctx.close()
+    assert min(ms) < 0.2, ms
+
+
 @pytest.mark.parametrize("n", [1, 2, 3, 7, 8, 33, 257])
 @pytest.mark.parametrize("rounds", [0, 3])
 def test_packed_traversal_finds_every_hit(n, rounds):

@@ -30,6 +30,7 @@
 #include <random>
 #include <stdexcept>
 #include <string>
+#include <type_traits>
 #include <utility>
 
 namespace vlrb {
@@ -547,29 +548,49 @@ __global__ void filmToRGBAKernel(Film film, FilmConst fc, float4* out) {
     }
 }
 
-// The launch's contributions into the film, one thread per pixel: it bins its
-// pixel's samples (path slots pixelCount apart, so a warp reads contiguous
-// contributions) into 16 FP64 strata of its own in shared memory, and the
-// warp then adds its 32 pixels' strata to the film in whole lines.  The
-// pixels have one writer, so there are no atomics.  `overwrite`: the first
-// launch of an accumulation stores instead of adding (no clear, no read).
-// `out`: the pixel's colour from the strata just written, XYZ / frames * (W*H)
-// -> Rec.709 D65, with `samples` added to the device frame count (the last
-// launch of a call that renders the whole film).
-// Bound by HBM: 32 B read per sample, 128 B written (and read when adding)
-// per pixel, 16 B of colour.  kPitch (odd) spreads the pixels' strata over
-// the banks.
+// The launch's contributions into the film.  `lanes` threads (a power of two
+// up to 32) share a pixel: each bins every lanes-th of its samples (path slots
+// pixelCount apart) into 16 FP64 strata of its own in shared memory, four
+// samples' loads at a time, and the warp then adds its pixels' strata, the
+// lanes' sums in order, to the film in whole lines.  The pixels have one
+// writer, so there are no atomics.  `overwrite`: the first launch of an
+// accumulation stores instead of adding (no clear, no read).  `out`: the
+// pixel's colour from the strata just written, XYZ / frames * (W*H) -> Rec.709
+// D65, with `samples` added to the device frame count (the last launch of a
+// call that renders the whole film).
+//
+// Bound by HBM where the pixels fill the GPU: 32 B read per sample, 128 B
+// written (and read when adding) per pixel, 16 B of colour.  With fewer pixels
+// a thread's samples are the chain, so the pixels are split (filmLanes).  With
+// one thread a pixel, one sample at a time, and now: 64 x 64 pixels, 512 samples a
+// launch, 633 -> 49 us; 32 x 32, 64: 62 -> 17; 512 x 512, 64: 199 -> 136; 1920 x
+// 1080, 1, adding to a film: 154 -> 114 (with its lines read ahead of the stores).
+// kPitch (odd) spreads the strata over the banks.
 constexpr int kFilmThreads = 128, kFilmPitch = kNumStrata + 1;
+
+__device__ __forceinline__ void binSample(double* strata, const float4 &contrib, float offset) {
+    const S4 c = toS4(contrib);
+    if (!c.allFinite()) return;
+    WLS wls;
+    wls.setOffset(offset);
+#pragma unroll
+    for (int w = 0; w < 4; ++w) strata[strataBin(wls.lambda[w])] += strataValue(c[w]);
+}
+
+template <bool kSplit, int kLoads, bool kAdd>
 __global__ void __launch_bounds__(kFilmThreads) filmResolveKernel(PathBuffers pb, Film film, FrameParams fp,
-                                                                  FilmConst fc, FilmResolve fr) {
+                                                                  FilmConst fc, FilmResolve fr, uint32_t samples,
+                                                                  uint32_t lanesArg) {
     __shared__ double sAcc[kFilmThreads * kFilmPitch];
     startDependent();
+    const uint32_t lanes = kSplit ? lanesArg : 1u;
     const uint32_t pixels = fp.width * fp.height;
-    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t lane = threadIdx.x & 31u, sub = lane % lanes;
+    const uint32_t warpPixels = 32u / lanes, blockPixels = kFilmThreads / lanes;
     double* mine = sAcc + threadIdx.x * kFilmPitch;
     double* warpAcc = sAcc + (threadIdx.x - lane) * kFilmPitch;
-    for (uint32_t base = blockIdx.x * kFilmThreads; base < pixels; base += gridDim.x * kFilmThreads) {
-        const uint32_t i = base + threadIdx.x;
+    for (uint32_t base = blockIdx.x * blockPixels; base < pixels; base += gridDim.x * blockPixels) {
+        const uint32_t i = base + threadIdx.x / lanes;
         const bool in = i < pixels;
         uint32_t fi = 0;
 #pragma unroll
@@ -577,38 +598,71 @@ __global__ void __launch_bounds__(kFilmThreads) filmResolveKernel(PathBuffers pb
         if (in) {
             const uint32_t pixel = pixelOfPath(i, fp.width, fp.height);
             fi = (pixel / fp.width) * fp.stride + pixel % fp.width;
-            for (uint32_t p = i; p < fp.numPaths; p += pixels) {
-                const S4 c = toS4(pb.contrib[p]);
-                if (!c.allFinite()) continue;
-                WLS wls;
-                wls.setOffset(__uint_as_float(pb.meta[p].w));
+            uint32_t s = sub;
+            for (; kLoads > 1 && s + (kLoads - 1) * lanes < samples; s += kLoads * lanes) {
+                float4 c[kLoads];
+                float offset[kLoads];
 #pragma unroll
-                for (int w = 0; w < 4; ++w) mine[strataBin(wls.lambda[w])] += strataValue(c[w]);
-            }
-        }
-        __syncwarp();
-        // two pixels' lines per step
-#pragma unroll
-        for (uint32_t r = 0; r < 16; ++r) {
-            const uint32_t j = 2 * r + (lane >> 4), k = lane & 15u;
-            const uint32_t fj = __shfl_sync(0xFFFFFFFFu, fi, j);
-            if (base + (threadIdx.x - lane) + j < pixels) {
-                double* dst = film.strata + static_cast<size_t>(fj) * kNumStrata + k;
-                double v = warpAcc[j * kFilmPitch + k];
-                if (!fr.overwrite) {
-                    v += *dst;
-                    warpAcc[j * kFilmPitch + k] = v;
+                for (uint32_t u = 0; u < kLoads; ++u) {
+                    const uint32_t p = i + (s + u * lanes) * pixels;
+                    c[u] = pb.contrib[p];
+                    offset[u] = __uint_as_float(pb.meta[p].w);
                 }
-                *dst = v;
+#pragma unroll
+                for (uint32_t u = 0; u < kLoads; ++u) binSample(mine, c[u], offset[u]);
+            }
+            for (; s < samples; s += lanes) {
+                const uint32_t p = i + s * pixels;
+                binSample(mine, pb.contrib[p], __uint_as_float(pb.meta[p].w));
             }
         }
         __syncwarp();
-        if (in && fr.out) {
+        // two pixels' lines per step; what the film holds is read ahead of the stores
+        const uint32_t warpBase = base + (threadIdx.x - lane) / lanes;
+        constexpr uint32_t kSteps = kSplit ? 8 : 16;
+        auto line = [&](uint32_t r) -> double* {
+            const uint32_t j = 2 * r + (lane >> 4);
+            const uint32_t fj = __shfl_sync(0xFFFFFFFFu, fi, (j * lanes) & 31u);
+            return j < warpPixels && warpBase + j < pixels
+                       ? film.strata + static_cast<size_t>(fj) * kNumStrata + (lane & 15u) : nullptr;
+        };
+        double held[kSteps];
+        if (kAdd) {
+#pragma unroll
+            for (uint32_t r = 0; r < kSteps; ++r) {
+                const double* src = line(r);
+                held[r] = src ? *src : 0.0;
+            }
+        }
+#pragma unroll
+        for (uint32_t r = 0; r < kSteps; ++r) {
+            double* dst = line(r);
+            if (!dst) continue;
+            double* sum = warpAcc + (2 * r + (lane >> 4)) * lanes * kFilmPitch + (lane & 15u);
+            double v = *sum;
+            if (kSplit)
+                for (uint32_t l = 1; l < lanes; ++l) v += sum[l * kFilmPitch];
+            if (kAdd) v += held[r];
+            if (kSplit || kAdd) *sum = v;
+            *dst = v;
+        }
+        __syncwarp();
+        if (in && sub == 0 && fr.out) {
             const uint32_t frames = (fr.overwriteFrames ? 0u : *film.frames) + fr.samples;
             fr.out[fi] = strataToRGBA(mine, fc, film.width * film.height, frames ? frames : 1u);
         }
         __syncwarp();
     }
+}
+
+// Threads per pixel of the film pass: as many as fill the GPU (eight blocks an
+// SM), with four samples' loads in flight each (256 x 256, 4 samples: 17 us with
+// one thread a pixel, 23 with four).
+inline uint32_t filmLanes(uint32_t pixels, uint32_t samples, int numSMs) {
+    const uint64_t wanted = static_cast<uint64_t>(numSMs) * 8 * kFilmThreads;
+    uint32_t lanes = 1;
+    while (lanes < 32 && 8 * lanes <= samples && static_cast<uint64_t>(pixels) * lanes < wanted) lanes *= 2;
+    return lanes;
 }
 
 // Adds this launch's per-bounce queue lengths to the running totals, and a
@@ -809,10 +863,22 @@ void ptRenderLaunch(const SceneGPU &scene, const PathBuffers &pb, const Film &fi
         T.end(stream);
     }
     T.begin(kStageFilm, stream, sizeof(PathBuffers) + sizeof(Film) + sizeof(FrameParams) + sizeof(FilmConst) +
-                                    sizeof(FilmResolve));
+                                    sizeof(FilmResolve) + 8);
     const uint32_t pixels = fp.width * fp.height;
-    launchChained(filmResolveKernel, std::min<uint32_t>((pixels + kFilmThreads - 1) / kFilmThreads, numSMs * 24u),
-                  kFilmThreads, chain, pb, film, fp, filmConst(), resolve);
+    const uint32_t samples = fp.numPaths / pixels;
+    const uint32_t lanes = filmLanes(pixels, samples, numSMs);
+    const uint32_t filmGrid = static_cast<uint32_t>(
+        std::min<uint64_t>((static_cast<uint64_t>(pixels) * lanes + kFilmThreads - 1) / kFilmThreads, numSMs * 24u));
+    auto filmPass = [&](auto add) {
+        constexpr bool kAdd = decltype(add)::value;
+        auto kernel = filmResolveKernel<false, 1, kAdd>;
+        if (lanes > 1) kernel = filmResolveKernel<true, 4, kAdd>;
+        else if (samples >= 4) kernel = filmResolveKernel<false, 4, kAdd>;
+        else if (samples >= 2) kernel = filmResolveKernel<false, 2, kAdd>;
+        launchChained(kernel, filmGrid, kFilmThreads, chain, pb, film, fp, filmConst(), resolve, samples, lanes);
+    };
+    if (resolve.overwrite) filmPass(std::false_type{});
+    else filmPass(std::true_type{});
     T.end(stream);
     T.begin(kStageFilm, stream, sizeof(PathBuffers) + 16 + sizeof(FilmResolve));
     launchChained(statsKernel, 1, 32, chain, pb, fp.maxPathLength, film.frames, resolve);
