@@ -324,10 +324,12 @@ def test_denoiser_matches_numpy(size):
     assert (off / scale).max() < 5e-3 and (off / scale).mean() < 1e-4
 
 
-@pytest.mark.parametrize("n", [1, 127, 128, 129, 256, 257, 113664, 113665, 113921])
+@pytest.mark.parametrize("n", [1, 127, 128, 129, 256, 257, 18944, 18945, 25000, 37888, 37889, 113664,
+                               113665, 113921])
 def test_guide_inference_tiles(n):
     """A query's network outputs do not depend on its tile: each prefix equals
-    the large batch bit for bit (113,664 rows fill the resident groups once)."""
+    the large batch bit for bit (18,944 rows are one tile per SM, 37,888 two, and
+    113,664 fill the resident groups once)."""
     from vlr_b200.guide import GuideNet
     rng = np.random.default_rng(3)
     net = GuideNet(12, seed=1)

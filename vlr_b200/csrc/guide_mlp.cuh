@@ -173,6 +173,17 @@ __device__ __forceinline__ void groupSync(uint32_t group) {
     else barrierSync<2>();
 }
 
+// CTAs for a known number of rows: one per tile up to one per SM, then two
+// tiles each.  (Every CTA two from the start: 300 rows 39 us, 5,000 31, 18,944 31;
+// so: 24, 22, 23.  From 25,000 rows the same.)
+inline uint32_t inferGrid(uint32_t rows, uint32_t numSMs) {
+    const uint32_t tiles = (rows + kRows - 1) / kRows;
+    const uint32_t paired = (tiles + kInferGroups - 1) / kInferGroups;
+    const uint32_t spread = tiles < numSMs ? tiles : numSMs;
+    const uint32_t wanted = paired > spread ? paired : spread;
+    return wanted < numSMs * kInferBlocksPerSM ? wanted : numSMs * kInferBlocksPerSM;
+}
+
 template <class Src, class Dst>
 __global__ void __launch_bounds__(kInferThreads, kInferBlocksPerSM) guideInferKernel(Net net, Src src, Dst dst,
                                                                                      uint32_t* err) {
@@ -196,8 +207,8 @@ __global__ void __launch_bounds__(kInferThreads, kInferBlocksPerSM) guideInferKe
     uint32_t phase = 0;
     const uint32_t n = src.count();
     bool ok = true;
-    for (uint32_t tile = blockIdx.x * kInferGroups + group; ok && tile * kRows < n;
-         tile += gridDim.x * kInferGroups) {
+    // a second tile shares a CTA only when every CTA has one
+    for (uint32_t tile = blockIdx.x + group * gridDim.x; ok && tile * kRows < n; tile += gridDim.x * kInferGroups) {
         const uint32_t row = tile * kRows + tid;
         float3 p;
         V3 wo, nrm;

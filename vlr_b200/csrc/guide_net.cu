@@ -168,10 +168,7 @@ void GuideNet::inferArrays(const float* pos, const float* wo, const float* nrm, 
     RawDst dst{ raw };
     auto kern = guideInferKernel<ArraySrc, RawDst>;
     ck(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kInferSmemBytes), "smem attr");
-    const uint32_t tiles = (n + kRows - 1) / kRows;
-    const uint32_t needed = (tiles + kInferGroups - 1) / kInferGroups;
-    const uint32_t resident = uint32_t(numSMs) * kInferBlocksPerSM;
-    const uint32_t grid = needed < resident ? needed : resident;
+    const uint32_t grid = inferGrid(n, uint32_t(numSMs));
     kern<<<grid, kInferThreads, kInferSmemBytes, stream>>>(net, src, dst, err);
     ck(cudaGetLastError(), "infer launch");
 }
