@@ -245,6 +245,76 @@ def test_host_copies_at_their_chunk_edges(ray_query, count):
     assert np.array_equal(_trace(v, rays[:count]).view(np.uint32), want[:count].view(np.uint32))
 
 
+def _memory(kind, a):
+    """A copy of array `a` in pinned, registered or device memory, and
+    its address."""
+    import torch
+    rt = torch.cuda.cudart()
+    if kind == "pinned":
+        t = torch.from_numpy(a.copy()).pin_memory()
+        return t, t.data_ptr()
+    if kind == "registered":
+        b = a.copy()
+        assert rt.cudaHostRegister(b.ctypes.data, b.nbytes, 0) in (0, rt.cudaError.success)
+        return b, b.ctypes.data
+    t = torch.from_numpy(a).cuda()
+    return t, t.data_ptr()
+
+
+@pytest.mark.parametrize("kind", ["pinned", "registered"])
+def test_host_copies_of_pinned_arrays(ray_query, kind):
+    import torch
+    v, rays, want = ray_query
+    hits = np.zeros((len(rays), 4), np.float32)
+    keep = [_memory(kind, a) for a in (v, rays, hits)]
+    assert V.lib().vlrbTraceRaysHost(ctypes.c_void_p(keep[0][1]), ctypes.c_uint32(len(v)), ctypes.c_uint32(3),
+                                     ctypes.c_void_p(keep[1][1]), ctypes.c_uint32(len(rays)), ctypes.c_uint32(0),
+                                     ctypes.c_void_p(keep[2][1]), None) == 0
+    out = np.asarray(keep[2][0])
+    assert np.array_equal(out.view(np.uint32), want.view(np.uint32))
+    if kind == "registered":
+        for k, _ in keep:
+            torch.cuda.cudart().cudaHostUnregister(k.ctypes.data)
+
+
+def test_pinned_arrays_are_not_staged(ray_query):
+    """A call's pinned arrays move at the link's rate: faster than pageable ones,
+    which a CPU has to copy first."""
+    import time
+    import torch
+    from vlr_b200 import guide
+    net = guide.GuideNet(14, seed=1)
+    n = 65536
+    rng = np.random.default_rng(2)
+    arrays = [rng.uniform(0, 1, (n, 3)).astype(np.float32) for _ in range(3)] + [np.zeros((n, 40), np.float32)]
+    pinned = [torch.from_numpy(a.copy()).pin_memory().numpy() for a in arrays]
+    P = lambda a: a.ctypes.data_as(ctypes.c_void_p)
+    best = []
+    for s in (arrays, pinned):
+        t = []
+        for _ in range(20):
+            t0 = time.perf_counter()
+            assert guide._api().vlrbGuideNetInferHost(net.h, n, *(P(a) for a in s)) == 0
+            t.append(time.perf_counter() - t0)
+        best.append(min(t))
+    net.close()
+    assert np.array_equal(arrays[3], pinned[3])
+    assert best[1] < best[0], best
+
+
+def test_device_memory_in_place_of_a_host_array_does_not_crash(ray_query):
+    """Whether the driver accepts it or not, the call answers (a CPU copy from a
+    device address ends the process)."""
+    v, rays, want = ray_query
+    keep = _memory("device", rays)
+    hits = np.zeros((len(rays), 4), np.float32)
+    P = lambda a: a.ctypes.data_as(ctypes.c_void_p)
+    r = V.lib().vlrbTraceRaysHost(P(v), ctypes.c_uint32(len(v)), ctypes.c_uint32(3), ctypes.c_void_p(keep[1]),
+                                  ctypes.c_uint32(len(rays)), ctypes.c_uint32(0), P(hits), None)
+    assert r == V.INTERNAL_ERROR or (r == 0 and np.array_equal(hits.view(np.uint32), want.view(np.uint32)))
+    assert np.array_equal(_trace(v, rays[:1000]).view(np.uint32), want[:1000].view(np.uint32))
+
+
 def test_host_calls_from_several_threads(ray_query):
     """Calls of different sizes at once, more of them than workspaces are kept."""
     from concurrent.futures import ThreadPoolExecutor

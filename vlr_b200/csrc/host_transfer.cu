@@ -60,6 +60,15 @@ namespace {
 std::mutex g_mutex;
 std::vector<HostWorkspace*> g_free;   // kept to the end of the process
 
+// Whether the CPU may stage the array: pinned memory moves by itself at the
+// link's rate, and device memory given as an array is the driver's to judge.
+bool pageable(const void* p) {
+    cudaPointerAttributes a{};
+    if (cudaPointerGetAttributes(&a, p) == cudaSuccess) return a.type == cudaMemoryTypeUnregistered;
+    cudaGetLastError();
+    return false;
+}
+
 // Runs work(worker) in this thread and, for a large copy, in kWorkers - 1
 // others; the first exception is rethrown when all have ended.
 template <class F>
@@ -152,7 +161,7 @@ HostTransfer::~HostTransfer() {
 void* HostTransfer::device() const { return w->dev; }
 
 void HostTransfer::upload(void* dst, const void* src, size_t bytes) {
-    if (bytes < kStaged) {
+    if (bytes < kStaged || !pageable(src)) {
         if (bytes) ck(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, nullptr), "upload");
         return;
     }
@@ -172,7 +181,7 @@ void HostTransfer::upload(void* dst, const void* src, size_t bytes) {
 }
 
 void HostTransfer::download(void* dst, const void* src, size_t bytes) {
-    if (bytes < kStaged) {
+    if (bytes < kStaged || !pageable(dst)) {
         if (bytes) ck(cudaMemcpy(dst, src, bytes, cudaMemcpyDeviceToHost), "download");
         return;
     }

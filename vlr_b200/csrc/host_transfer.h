@@ -32,7 +32,9 @@ public:
     HostTransfer &operator=(const HostTransfer &) = delete;
 
     void* device() const;
-    // Enqueues the copy; returns once `src` has been read.
+    // Enqueues the copy.  `src` may be read until the next download or the end of
+    // this object, and must stay as it is until then.  Pageable arrays are staged;
+    // any other memory goes to the driver as it is.
     void upload(void* dst, const void* src, size_t bytes);
     // Returns once `dst` holds the bytes the stream's earlier work left at `src`.
     void download(void* dst, const void* src, size_t bytes);
