@@ -326,6 +326,32 @@ def test_host_calls_from_several_threads(ray_query):
         assert np.array_equal(g.view(np.uint32), want[a:a + n].view(np.uint32))
 
 
+def test_many_callers_do_not_slow_each_other(ray_query):
+    """Small calls of eight threads, per call, against those of one: the work of
+    all is on one stream, so a call takes as long as alone (a half for scatter)
+    unless the calls beyond the kept workspaces make and undo their own."""
+    import time
+    from concurrent.futures import ThreadPoolExecutor
+    v, rays, _ = ray_query
+    v, rays = v[:500].copy(), rays[:1000].copy()
+
+    def per_call(pool, k):
+        def calls():
+            for _ in range(6):
+                _trace(v, rays)
+        best = []
+        for _ in range(6):
+            t0 = time.perf_counter()
+            for f in [pool.submit(calls) for _ in range(k)]:
+                f.result()
+            best.append((time.perf_counter() - t0) / (6 * k))
+        return min(best)
+
+    with ThreadPoolExecutor(8) as pool:
+        alone, together = per_call(pool, 1), per_call(pool, 8)
+    assert together < 1.5 * alone, (together, alone)
+
+
 def _atrous(color, albedo, normal):
     """The denoiser in numpy (float64, guides rounded to halves as stored)."""
     eps = 1e-3

@@ -5,6 +5,8 @@
 #include <algorithm>
 #include <atomic>
 #include <cstring>
+#include <exception>
+#include <map>
 #include <mutex>
 #include <stdexcept>
 #include <string>
@@ -22,7 +24,12 @@ namespace {
 constexpr int kWorkers = 4, kSlotsPerWorker = 2, kSlots = kWorkers * kSlotsPerWorker;
 constexpr size_t kChunk = size_t(1) << 20;
 constexpr size_t kStaged = size_t(256) << 10, kThreaded = size_t(2) << 20;
-constexpr size_t kKept = 2, kKeptBytes = size_t(256) << 20;
+// Rings and device blocks kept per device.  A ring takes milliseconds to make,
+// so callers beyond the rings' number copy through the driver instead of
+// making more (eight callers of 1,000 rays each: 2,470 us a call with rings of
+// their own, 810 so).
+constexpr int kRings = 2;
+constexpr size_t kKeptBlocks = 8, kKeptBytes = size_t(256) << 20;
 
 void ck(cudaError_t e, const char* what) {
     if (e != cudaSuccess) throw std::runtime_error(std::string("host transfer ") + what + ": " + cudaGetErrorString(e));
@@ -30,19 +37,16 @@ void ck(cudaError_t e, const char* what) {
 
 } // namespace
 
-struct HostWorkspace {
+struct HostRing {
     int device = 0;
-    void* dev = nullptr;
-    size_t devBytes = 0;
     char* pinned = nullptr;
     cudaEvent_t done[kSlots] = {};
     bool used[kSlots] = {};
 
-    ~HostWorkspace() {
+    ~HostRing() {
         for (cudaEvent_t e : done)
             if (e) cudaEventDestroy(e);
         if (pinned) cudaFreeHost(pinned);
-        if (dev) cudaFree(dev);
     }
     char* slot(int s) const { return pinned + size_t(s) * kChunk; }
     void wait(int s) {
@@ -57,8 +61,89 @@ struct HostWorkspace {
 
 namespace {
 
+struct DeviceBlock {
+    int device;
+    void* p;
+    size_t bytes;
+};
+
+// Idle ones; they stay to the end of the process.
 std::mutex g_mutex;
-std::vector<HostWorkspace*> g_free;   // kept to the end of the process
+std::vector<DeviceBlock> g_blocks;
+std::vector<HostRing*> g_rings;
+std::map<int, int> g_ringsMade;   // per device, idle or borrowed
+
+// The smallest idle block of at least `bytes`.
+bool takeBlock(int device, size_t bytes, DeviceBlock* out) {
+    std::lock_guard<std::mutex> lock(g_mutex);
+    size_t best = g_blocks.size();
+    for (size_t i = 0; i < g_blocks.size(); ++i)
+        if (g_blocks[i].device == device && g_blocks[i].bytes >= bytes &&
+            (best == g_blocks.size() || g_blocks[i].bytes < g_blocks[best].bytes))
+            best = i;
+    if (best == g_blocks.size()) return false;
+    *out = g_blocks[best];
+    g_blocks.erase(g_blocks.begin() + static_cast<std::ptrdiff_t>(best));
+    return true;
+}
+
+// Keeps an idle block, in place of smaller ones where the limits ask for it.
+void keepBlock(const DeviceBlock &block) {
+    std::vector<void*> dropped;
+    {
+        std::lock_guard<std::mutex> lock(g_mutex);
+        size_t count = 0, bytes = 0;
+        for (const DeviceBlock &k : g_blocks)
+            if (k.device == block.device) { ++count; bytes += k.bytes; }
+        while (block.bytes <= kKeptBytes && (count + 1 > kKeptBlocks || bytes + block.bytes > kKeptBytes)) {
+            auto least = g_blocks.end();
+            for (auto i = g_blocks.begin(); i != g_blocks.end(); ++i)
+                if (i->device == block.device && i->bytes < block.bytes && (least == g_blocks.end() || i->bytes < least->bytes))
+                    least = i;
+            if (least == g_blocks.end()) break;
+            --count;
+            bytes -= least->bytes;
+            dropped.push_back(least->p);
+            g_blocks.erase(least);
+        }
+        if (count + 1 <= kKeptBlocks && bytes + block.bytes <= kKeptBytes) g_blocks.push_back(block);
+        else dropped.push_back(block.p);
+    }
+    for (void* p : dropped) cudaFree(p);
+}
+
+// An idle ring, a new one, or null: the caller then copies through the driver.
+HostRing* takeRing(int device) {
+    {
+        std::lock_guard<std::mutex> lock(g_mutex);
+        for (size_t i = 0; i < g_rings.size(); ++i)
+            if (g_rings[i]->device == device) {
+                HostRing* r = g_rings[i];
+                g_rings.erase(g_rings.begin() + static_cast<std::ptrdiff_t>(i));
+                return r;
+            }
+        if (g_ringsMade[device] >= kRings) return nullptr;
+        ++g_ringsMade[device];
+    }
+    HostRing* r = new HostRing;
+    r->device = device;
+    bool ok = cudaMallocHost(reinterpret_cast<void**>(&r->pinned), kSlots * kChunk) == cudaSuccess;
+    for (int i = 0; ok && i < kSlots; ++i)
+        ok = cudaEventCreateWithFlags(&r->done[i], cudaEventDisableTiming) == cudaSuccess;
+    if (ok) return r;
+    cudaGetLastError();
+    delete r;
+    std::lock_guard<std::mutex> lock(g_mutex);
+    --g_ringsMade[device];
+    return nullptr;
+}
+
+void returnRing(HostRing* r, bool idle) {
+    std::lock_guard<std::mutex> lock(g_mutex);
+    if (idle) { g_rings.push_back(r); return; }
+    --g_ringsMade[r->device];
+    delete r;
+}
 
 // Whether the CPU may stage the array: pinned memory moves by itself at the
 // link's rate, and device memory given as an array is the driver's to judge.
@@ -101,72 +186,43 @@ void runWorkers(int device, size_t bytes, F work) {
 
 } // namespace
 
-HostTransfer::HostTransfer(size_t deviceBytes) : w(nullptr) {
-    int device = 0;
-    ck(cudaGetDevice(&device), "device");
-    {
-        // the smallest kept workspace that is large enough, else the largest
-        std::lock_guard<std::mutex> lock(g_mutex);
-        size_t best = g_free.size();
-        for (size_t i = 0; i < g_free.size(); ++i) {
-            if (g_free[i]->device != device) continue;
-            if (best == g_free.size()) { best = i; continue; }
-            const size_t a = g_free[i]->devBytes, b = g_free[best]->devBytes;
-            if (a >= deviceBytes ? (b < deviceBytes || a < b) : (b < deviceBytes && a > b)) best = i;
-        }
-        if (best < g_free.size()) {
-            w = g_free[best];
-            g_free.erase(g_free.begin() + static_cast<std::ptrdiff_t>(best));
-        }
+HostTransfer::HostTransfer(size_t deviceBytes) {
+    ck(cudaGetDevice(&deviceIndex), "device");
+    DeviceBlock block{ deviceIndex, nullptr, deviceBytes };
+    if (!takeBlock(deviceIndex, deviceBytes, &block)) {
+        const cudaError_t e = cudaMalloc(&block.p, deviceBytes);
+        if (e != cudaSuccess) cudaGetLastError();
+        ck(e, "workspace");
     }
-    if (!w) {
-        w = new HostWorkspace;
-        w->device = device;
-    }
-    try {
-        if (!w->pinned) {
-            ck(cudaMallocHost(reinterpret_cast<void**>(&w->pinned), kSlots * kChunk), "pinned memory");
-            for (cudaEvent_t &e : w->done) ck(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "event");
-        }
-        if (w->devBytes < deviceBytes) {
-            if (w->dev) cudaFree(w->dev);
-            w->dev = nullptr;
-            w->devBytes = 0;
-            ck(cudaMalloc(&w->dev, deviceBytes), "workspace");
-            w->devBytes = deviceBytes;
-        }
-    }
-    catch (...) {
-        delete w;
-        cudaGetLastError();
-        throw;
-    }
+    dev = block.p;
+    devBytes = block.bytes;
 }
 
 HostTransfer::~HostTransfer() {
-    // nothing of this call may still use the buffers when another takes them
+    // nothing of this call may still use what another takes
     const bool idle = cudaStreamSynchronize(nullptr) == cudaSuccess;
-    if (idle && w->devBytes <= kKeptBytes) {
-        std::lock_guard<std::mutex> lock(g_mutex);
-        size_t kept = 0;
-        for (const HostWorkspace* f : g_free) kept += f->device == w->device;
-        if (kept < kKept) {
-            g_free.push_back(w);
-            return;
-        }
-    }
-    delete w;
+    if (ring) returnRing(ring, idle);
+    if (idle) keepBlock(DeviceBlock{ deviceIndex, dev, devBytes });
+    else cudaFree(dev);
 }
 
-void* HostTransfer::device() const { return w->dev; }
+void* HostTransfer::device() const { return dev; }
+
+bool HostTransfer::staged(const void* array, size_t bytes) {
+    if (bytes < kStaged || !pageable(array)) return false;
+    if (!ring && !ringAsked) ring = takeRing(deviceIndex);
+    ringAsked = true;
+    return ring != nullptr;
+}
 
 void HostTransfer::upload(void* dst, const void* src, size_t bytes) {
-    if (bytes < kStaged || !pageable(src)) {
+    if (!staged(src, bytes)) {
         if (bytes) ck(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, nullptr), "upload");
         return;
     }
+    HostRing* const w = ring;
     std::atomic<size_t> next{ 0 };
-    runWorkers(w->device, bytes, [&](int worker) {
+    runWorkers(deviceIndex, bytes, [&](int worker) {
         for (int turn = 0;; ++turn) {
             const size_t at = next.fetch_add(1) * kChunk;
             if (at >= bytes) return;
@@ -181,12 +237,13 @@ void HostTransfer::upload(void* dst, const void* src, size_t bytes) {
 }
 
 void HostTransfer::download(void* dst, const void* src, size_t bytes) {
-    if (bytes < kStaged || !pageable(dst)) {
+    if (!staged(dst, bytes)) {
         if (bytes) ck(cudaMemcpy(dst, src, bytes, cudaMemcpyDeviceToHost), "download");
         return;
     }
+    HostRing* const w = ring;
     std::atomic<size_t> next{ 0 };
-    runWorkers(w->device, bytes, [&](int worker) {
+    runWorkers(deviceIndex, bytes, [&](int worker) {
         size_t pendingAt = 0, pendingLen = 0;
         int pending = -1;
         auto drain = [&] {

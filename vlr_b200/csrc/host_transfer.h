@@ -3,16 +3,17 @@
 // Those calls were bound by what surrounds their kernels: device allocations
 // and frees made and undone every call, and copies between pageable memory and
 // the device, which the driver stages through one thread.  A HostTransfer
-// borrows a workspace for one call: a device buffer kept from earlier calls
-// and a ring of pinned slots that several threads fill or drain while the copy
-// engine works on the others.  One million rays against 20,022 triangles (32 MB
-// in, 16 MB out, the hierarchy built on the way): 8.4 -> 5.4 ms; the hierarchy of
-// 150,001 triangles: 4.4 -> 2.7 ms; 65,536 queries and gradients of the guiding
-// network: 4.0 -> 2.5 ms.
+// borrows for one call a device block kept from earlier calls and, once it has
+// a large pageable array to move, a ring of pinned slots that several threads
+// fill or drain while the copy engine works on the others.  One million rays
+// against 20,022 triangles (32 MB in, 16 MB out, the hierarchy built on the way):
+// 8.4 -> 5.4 ms; the hierarchy of 150,001 triangles: 4.4 -> 2.7 ms; 65,536
+// queries and gradients of the guiding network: 4.0 -> 2.5 ms.
 //
-// Workspaces are per device; a call has one to itself, so calls from several
-// threads run side by side.  At most kKept of them stay with the process, with
-// device buffers of at most kKeptBytes; others are freed when their call ends.
+// Blocks and rings are per device; a call has its own, so calls from several
+// threads run side by side.  What is kept is bounded: two rings (calls that find
+// both in use copy through the driver), and at most eight blocks of 256 MB in
+// all; a larger block is freed when its call ends.
 // All work is on the legacy default stream, which orders it after other
 // blocking streams' work as cudaMemcpy does.
 #pragma once
@@ -21,7 +22,7 @@
 
 namespace vlrb {
 
-struct HostWorkspace;
+struct HostRing;
 
 class HostTransfer {
 public:
@@ -40,7 +41,13 @@ public:
     void download(void* dst, const void* src, size_t bytes);
 
 private:
-    HostWorkspace* w;
+    bool staged(const void* array, size_t bytes);
+
+    int deviceIndex = 0;
+    void* dev = nullptr;
+    size_t devBytes = 0;
+    HostRing* ring = nullptr;
+    bool ringAsked = false;
 };
 
 } // namespace vlrb
