@@ -1,5 +1,6 @@
 #include "host_transfer.h"
 
+#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -24,7 +25,7 @@ namespace {
 constexpr int kWorkers = 4, kSlotsPerWorker = 2, kSlots = kWorkers * kSlotsPerWorker;
 constexpr size_t kChunk = size_t(1) << 20;
 constexpr size_t kStaged = size_t(256) << 10, kThreaded = size_t(2) << 20;
-// Rings and device blocks kept per device.  A ring takes milliseconds to make,
+// Rings and device blocks kept per CUDA context.  A ring takes milliseconds to make,
 // so callers beyond the rings' number copy through the driver instead of
 // making more (eight callers of 1,000 rays each: 2,470 us a call with rings of
 // their own, 810 so).
@@ -37,8 +38,16 @@ void ck(cudaError_t e, const char* what) {
 
 } // namespace
 
+// The CUDA context all handles and addresses belong to.  The id is never used
+// again in a process: after cudaDeviceReset a device's primary context has the
+// same handle and another id, and what was kept of the old one is gone with it.
+struct CudaContext {
+    CUcontext handle = nullptr;
+    unsigned long long id = 0;
+};
+
 struct HostRing {
-    int device = 0;
+    CudaContext context;
     char* pinned = nullptr;
     cudaEvent_t done[kSlots] = {};
     bool used[kSlots] = {};
@@ -62,23 +71,75 @@ struct HostRing {
 namespace {
 
 struct DeviceBlock {
-    int device;
+    CudaContext context;
     void* p;
     size_t bytes;
 };
 
-// Idle ones; they stay to the end of the process.
+// The driver's calls through the runtime (no link-time libcuda dependency).
+struct Driver {
+    CUresult (*getCurrent)(CUcontext*) = nullptr;
+    CUresult (*setCurrent)(CUcontext) = nullptr;
+    CUresult (*getId)(CUcontext, unsigned long long*) = nullptr;
+};
+template <class F>
+void driverEntry(const char* name, F* fn) {
+    void* p = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    ck(cudaGetDriverEntryPoint(name, &p, cudaEnableDefault, &q), name);
+    if (!p) throw std::runtime_error(std::string("host transfer: no ") + name);
+    *fn = reinterpret_cast<F>(p);
+}
+const Driver &driver() {
+    static const Driver d = [] {
+        Driver r;
+        driverEntry("cuCtxGetCurrent", &r.getCurrent);
+        driverEntry("cuCtxSetCurrent", &r.setCurrent);
+        driverEntry("cuCtxGetId", &r.getId);
+        return r;
+    }();
+    return d;
+}
+
+CudaContext currentContext() {
+    ck(cudaFree(nullptr), "context");   // makes the device's primary context if none is current
+    CudaContext c;
+    if (driver().getCurrent(&c.handle) != CUDA_SUCCESS || !c.handle ||
+        driver().getId(c.handle, &c.id) != CUDA_SUCCESS)
+        throw std::runtime_error("host transfer: no CUDA context");
+    return c;
+}
+
+// Idle ones.
 std::mutex g_mutex;
 std::vector<DeviceBlock> g_blocks;
 std::vector<HostRing*> g_rings;
-std::map<int, int> g_ringsMade;   // per device, idle or borrowed
+std::map<unsigned long long, int> g_ringsMade;   // per context, idle or borrowed
+
+// Forgets what was kept of a context that is gone: its handle is `now`'s, its
+// id is not.  (With the mutex held.)
+void forgetGone(const CudaContext &now) {
+    auto gone = [&](const CudaContext &c) { return c.handle == now.handle && c.id != now.id; };
+    g_blocks.erase(std::remove_if(g_blocks.begin(), g_blocks.end(), [&](const DeviceBlock &b) { return gone(b.context); }),
+                   g_blocks.end());
+    for (HostRing* &r : g_rings)
+        if (gone(r->context)) {
+            g_ringsMade.erase(r->context.id);
+            r->pinned = nullptr;
+            for (cudaEvent_t &e : r->done) e = nullptr;
+            delete r;
+            r = nullptr;
+        }
+    g_rings.erase(std::remove(g_rings.begin(), g_rings.end(), nullptr), g_rings.end());
+}
 
 // The smallest idle block of at least `bytes`.
-bool takeBlock(int device, size_t bytes, DeviceBlock* out) {
+bool takeBlock(const CudaContext &context, size_t bytes, DeviceBlock* out) {
     std::lock_guard<std::mutex> lock(g_mutex);
+    forgetGone(context);
     size_t best = g_blocks.size();
     for (size_t i = 0; i < g_blocks.size(); ++i)
-        if (g_blocks[i].device == device && g_blocks[i].bytes >= bytes &&
+        if (g_blocks[i].context.id == context.id && g_blocks[i].bytes >= bytes &&
             (best == g_blocks.size() || g_blocks[i].bytes < g_blocks[best].bytes))
             best = i;
     if (best == g_blocks.size()) return false;
@@ -94,11 +155,12 @@ void keepBlock(const DeviceBlock &block) {
         std::lock_guard<std::mutex> lock(g_mutex);
         size_t count = 0, bytes = 0;
         for (const DeviceBlock &k : g_blocks)
-            if (k.device == block.device) { ++count; bytes += k.bytes; }
+            if (k.context.id == block.context.id) { ++count; bytes += k.bytes; }
         while (block.bytes <= kKeptBytes && (count + 1 > kKeptBlocks || bytes + block.bytes > kKeptBytes)) {
             auto least = g_blocks.end();
             for (auto i = g_blocks.begin(); i != g_blocks.end(); ++i)
-                if (i->device == block.device && i->bytes < block.bytes && (least == g_blocks.end() || i->bytes < least->bytes))
+                if (i->context.id == block.context.id && i->bytes < block.bytes &&
+                    (least == g_blocks.end() || i->bytes < least->bytes))
                     least = i;
             if (least == g_blocks.end()) break;
             --count;
@@ -113,20 +175,20 @@ void keepBlock(const DeviceBlock &block) {
 }
 
 // An idle ring, a new one, or null: the caller then copies through the driver.
-HostRing* takeRing(int device) {
+HostRing* takeRing(const CudaContext &context) {
     {
         std::lock_guard<std::mutex> lock(g_mutex);
         for (size_t i = 0; i < g_rings.size(); ++i)
-            if (g_rings[i]->device == device) {
+            if (g_rings[i]->context.id == context.id) {
                 HostRing* r = g_rings[i];
                 g_rings.erase(g_rings.begin() + static_cast<std::ptrdiff_t>(i));
                 return r;
             }
-        if (g_ringsMade[device] >= kRings) return nullptr;
-        ++g_ringsMade[device];
+        if (g_ringsMade[context.id] >= kRings) return nullptr;
+        ++g_ringsMade[context.id];
     }
     HostRing* r = new HostRing;
-    r->device = device;
+    r->context = context;
     bool ok = cudaMallocHost(reinterpret_cast<void**>(&r->pinned), kSlots * kChunk) == cudaSuccess;
     for (int i = 0; ok && i < kSlots; ++i)
         ok = cudaEventCreateWithFlags(&r->done[i], cudaEventDisableTiming) == cudaSuccess;
@@ -134,14 +196,14 @@ HostRing* takeRing(int device) {
     cudaGetLastError();
     delete r;
     std::lock_guard<std::mutex> lock(g_mutex);
-    --g_ringsMade[device];
+    --g_ringsMade[context.id];
     return nullptr;
 }
 
 void returnRing(HostRing* r, bool idle) {
     std::lock_guard<std::mutex> lock(g_mutex);
     if (idle) { g_rings.push_back(r); return; }
-    --g_ringsMade[r->device];
+    --g_ringsMade[r->context.id];
     delete r;
 }
 
@@ -157,13 +219,14 @@ bool pageable(const void* p) {
 // Runs work(worker) in this thread and, for a large copy, in kWorkers - 1
 // others; the first exception is rethrown when all have ended.
 template <class F>
-void runWorkers(int device, size_t bytes, F work) {
+void runWorkers(const CudaContext &context, size_t bytes, F work) {
     int n = bytes < kThreaded ? 1 : std::min<int>(kWorkers, static_cast<int>((bytes + kChunk - 1) / kChunk));
     n = std::min<int>(n, std::max<int>(1, static_cast<int>(std::thread::hardware_concurrency()) / 2));
     std::exception_ptr failed[kWorkers];
     auto guarded = [&](int worker) {
         try {
-            if (worker > 0) ck(cudaSetDevice(device), "device");
+            if (worker > 0 && driver().setCurrent(context.handle) != CUDA_SUCCESS)
+                throw std::runtime_error("host transfer: worker without the caller's context");
             work(worker);
         }
         catch (...) {
@@ -187,9 +250,11 @@ void runWorkers(int device, size_t bytes, F work) {
 } // namespace
 
 HostTransfer::HostTransfer(size_t deviceBytes) {
-    ck(cudaGetDevice(&deviceIndex), "device");
-    DeviceBlock block{ deviceIndex, nullptr, deviceBytes };
-    if (!takeBlock(deviceIndex, deviceBytes, &block)) {
+    const CudaContext context = currentContext();
+    contextHandle = context.handle;
+    contextId = context.id;
+    DeviceBlock block{ context, nullptr, deviceBytes };
+    if (!takeBlock(context, deviceBytes, &block)) {
         const cudaError_t e = cudaMalloc(&block.p, deviceBytes);
         if (e != cudaSuccess) cudaGetLastError();
         ck(e, "workspace");
@@ -202,7 +267,7 @@ HostTransfer::~HostTransfer() {
     // nothing of this call may still use what another takes
     const bool idle = cudaStreamSynchronize(nullptr) == cudaSuccess;
     if (ring) returnRing(ring, idle);
-    if (idle) keepBlock(DeviceBlock{ deviceIndex, dev, devBytes });
+    if (idle) keepBlock(DeviceBlock{ { contextHandle, contextId }, dev, devBytes });
     else cudaFree(dev);
 }
 
@@ -210,7 +275,7 @@ void* HostTransfer::device() const { return dev; }
 
 bool HostTransfer::staged(const void* array, size_t bytes) {
     if (bytes < kStaged || !pageable(array)) return false;
-    if (!ring && !ringAsked) ring = takeRing(deviceIndex);
+    if (!ring && !ringAsked) ring = takeRing({ contextHandle, contextId });
     ringAsked = true;
     return ring != nullptr;
 }
@@ -222,7 +287,7 @@ void HostTransfer::upload(void* dst, const void* src, size_t bytes) {
     }
     HostRing* const w = ring;
     std::atomic<size_t> next{ 0 };
-    runWorkers(deviceIndex, bytes, [&](int worker) {
+    runWorkers(w->context, bytes, [&](int worker) {
         for (int turn = 0;; ++turn) {
             const size_t at = next.fetch_add(1) * kChunk;
             if (at >= bytes) return;
@@ -243,7 +308,7 @@ void HostTransfer::download(void* dst, const void* src, size_t bytes) {
     }
     HostRing* const w = ring;
     std::atomic<size_t> next{ 0 };
-    runWorkers(deviceIndex, bytes, [&](int worker) {
+    runWorkers(w->context, bytes, [&](int worker) {
         size_t pendingAt = 0, pendingLen = 0;
         int pending = -1;
         auto drain = [&] {

@@ -10,8 +10,9 @@
 // 8.4 -> 5.4 ms; the hierarchy of 150,001 triangles: 4.4 -> 2.7 ms; 65,536
 // queries and gradients of the guiding network: 4.0 -> 2.5 ms.
 //
-// Blocks and rings are per device; a call has its own, so calls from several
-// threads run side by side.  What is kept is bounded: two rings (calls that find
+// Blocks and rings belong to a CUDA context, and are forgotten when it is gone
+// (cudaDeviceReset); a call has its own, so calls from several threads run side by
+// side.  What is kept is bounded: two rings (calls that find
 // both in use copy through the driver), and at most eight blocks of 256 MB in
 // all; a larger block is freed when its call ends.
 // All work is on the legacy default stream, which orders it after other
@@ -19,6 +20,8 @@
 #pragma once
 
 #include <cstddef>
+
+struct CUctx_st;
 
 namespace vlrb {
 
@@ -43,7 +46,8 @@ public:
 private:
     bool staged(const void* array, size_t bytes);
 
-    int deviceIndex = 0;
+    CUctx_st* contextHandle = nullptr;
+    unsigned long long contextId = 0;
     void* dev = nullptr;
     size_t devBytes = 0;
     HostRing* ring = nullptr;
