@@ -352,6 +352,49 @@ def test_many_callers_do_not_slow_each_other(ray_query):
     assert together < 1.5 * alone, (together, alone)
 
 
+def test_kept_memory_gives_way(ray_query):
+    """What host calls keep is released when the device has no memory left: with
+    it a larger call fits, and so does a renderer; and it goes with the last
+    context."""
+    import torch
+    MB = 1 << 20
+
+    def build(n):
+        v = np.random.default_rng(n).uniform(0, 1, (n, 9)).astype(np.float32)
+        out = [np.zeros(n, np.uint32), np.zeros(n, np.uint32), np.zeros(2 * n - 2, np.int32),
+               np.zeros(6 * n - 6, np.float32)]
+        return V.lib().vlrbBvhBuildHost(*(a.ctypes.data_as(ctypes.c_void_p) for a in [v]), ctypes.c_uint32(n),
+                                        *(a.ctypes.data_as(ctypes.c_void_p) for a in out), None)
+
+    def free():
+        return torch.cuda.mem_get_info()[0]
+
+    def all_but(left):
+        torch.cuda.synchronize()
+        hog = torch.empty(free() - left, dtype=torch.uint8, device="cuda")
+        assert free() < left + 8 * MB
+        return hog
+
+    torch.cuda.empty_cache()
+    ctx, cam, keep = _render_context(32, 32)
+    assert build(600000) == 0                    # about 150 MB are kept
+    hog = all_but(100 * MB)
+    assert build(800000) == 0                    # needs about 200
+    del hog
+    torch.cuda.empty_cache()
+    hog = all_but(100 * MB)
+    ctx.setOptions(max_paths_in_flight=1 << 19)
+    ctx.render_samples(cam, True, 512)           # about 120 MB of path state
+    del hog
+    torch.cuda.empty_cache()
+    assert build(600000) == 0
+    held = free()
+    ctx.close()
+    del keep
+    assert free() > held + 140 * MB
+    assert build(600000) == 0
+
+
 def _atrous(color, albedo, normal):
     """The denoiser in numpy (float64, guides rounded to halves as stored)."""
     eps = 1e-3

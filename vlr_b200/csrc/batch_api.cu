@@ -72,7 +72,7 @@ static cudaError_t growDevice(void** p, size_t* have, size_t want) {
     if (*p) cudaFree(*p);
     *p = nullptr;
     *have = 0;
-    const cudaError_t e = cudaMalloc(p, want);
+    const cudaError_t e = vlrb::deviceMalloc(p, want);
     if (e == cudaSuccess) *have = want;
     return e;
 }

@@ -9,11 +9,13 @@
 // reference's probabilities: emitting instances (environment first) and
 // emitting material groups are chosen uniformly, triangles by area.
 #include "context.cuh"
+#include "host_transfer.h"
 #include "lbvh_build.h"
 #include "tables.cuh"
 #include "bpt.cuh"
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstring>
 #include <functional>
@@ -34,6 +36,19 @@ namespace {
 void ck(cudaError_t e, const char* what) {
     if (e != cudaSuccess) throw std::runtime_error(std::string(what) + ": " + cudaGetErrorString(e));
 }
+
+// cudaMallocArray, as deviceMalloc.
+cudaError_t arrayMalloc(cudaArray_t* a, const cudaChannelFormatDesc &desc, size_t w, size_t h) {
+    cudaError_t e = cudaMallocArray(a, &desc, w, h);
+    if (e != cudaErrorMemoryAllocation) return e;
+    cudaGetLastError();
+    releaseHostTransfers();
+    e = cudaMallocArray(a, &desc, w, h);
+    if (e != cudaSuccess) cudaGetLastError();
+    return e;
+}
+
+std::atomic<int> g_contexts{ 0 };
 
 // Column-major 4x4 helpers.
 void matMul(const float a[16], const float b[16], float out[16]) {
@@ -112,7 +127,7 @@ void DeviceBuffer::release() {
 void DeviceBuffer::resize(size_t b) {
     if (b <= bytes && ptr) return;
     release();
-    ck(cudaMalloc(&ptr, b > 0 ? b : 1), "cudaMalloc");
+    ck(deviceMalloc(&ptr, b > 0 ? b : 1), "cudaMalloc");
     bytes = b;
 }
 
@@ -123,6 +138,7 @@ Context::Context(CUcontext cu, bool log) : Object(Kind::Context), cuContext(cu),
     ck(cudaDeviceGetAttribute(&numSMs, cudaDevAttrMultiProcessorCount, device), "SM count");
     ck(cudaMallocHost(reinterpret_cast<void**>(&hostCounters), (kMaxBounces + 1) * kCountersPerBounce * 4),
        "pinned counters");
+    ++g_contexts;
 }
 
 Context::~Context() {
@@ -130,6 +146,7 @@ Context::~Context() {
     objects.clear();
     if (outArray) cudaFreeArray(reinterpret_cast<cudaArray_t>(outArray));
     if (hostCounters) cudaFreeHost(hostCounters);
+    if (--g_contexts == 0) releaseHostTransfers();
 }
 
 void Context::destroy(Object* o) {
@@ -169,7 +186,7 @@ CUarray Context::outputArray() {
     if (!outArray && width > 0) {
         cudaChannelFormatDesc desc = cudaCreateChannelDesc<float4>();
         cudaArray_t a = nullptr;
-        ck(cudaMallocArray(&a, &desc, width, height), "cudaMallocArray");
+        ck(arrayMalloc(&a, desc, width, height), "cudaMallocArray");
         outArray = reinterpret_cast<CUarray>(a);
     }
     if (outArray)
@@ -654,7 +671,7 @@ void Context::buildScene(cudaStream_t stream) {
             if (it != texIndex.end()) return it->second;
             auto st = std::make_unique<SceneTexture>();
             const cudaChannelFormatDesc ch = cudaCreateChannelDesc<float4>();
-            ck(cudaMallocArray(&st->array, &ch, img->width, img->height), "texture array");
+            ck(arrayMalloc(&st->array, ch, img->width, img->height), "texture array");
             ck(cudaMemcpy2DToArray(st->array, 0, 0, img->rgba.data(), size_t(img->width) * 16,
                                    size_t(img->width) * 16, img->height, cudaMemcpyHostToDevice),
                "texture upload");
@@ -864,7 +881,7 @@ void Context::buildScene(cudaStream_t stream) {
             // the (u, v, s) image in a texture object the renderers fetch bilinearly
             auto st = std::make_unique<SceneTexture>();
             cudaChannelFormatDesc cd = cudaCreateChannelDescHalf4();
-            ck(cudaMallocArray(&st->array, &cd, w, h), "env array");
+            ck(arrayMalloc(&st->array, cd, w, h), "env array");
             ck(cudaMemcpy2DToArray(st->array, 0, 0, uvs.data(), size_t(w) * 8, size_t(w) * 8, h,
                                    cudaMemcpyHostToDevice), "env upload");
             cudaResourceDesc rd{};

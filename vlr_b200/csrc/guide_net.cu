@@ -99,7 +99,7 @@ GuideNet::GuideNet(uint32_t log2Table, uint64_t seed) {
     const size_t g = gridFloats();
     const size_t bytes = 4 * g * 4 + 4 * size_t(kNumWeights) * 4 + kWeightTileBytes + 256 +
                          size_t(numSMs) * kDwSlabFloats * 4 + 64;
-    ck(cudaMalloc(&mem, bytes), "alloc");
+    ck(deviceMalloc(&mem, bytes), "alloc");
     char* p = static_cast<char*>(mem);
     auto take = [&](size_t b) { char* r = p; p += (b + 255) & ~size_t(255); return r; };
     net.grid = reinterpret_cast<float*>(take(g * 4));

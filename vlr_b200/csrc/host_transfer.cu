@@ -249,15 +249,49 @@ void runWorkers(const CudaContext &context, size_t bytes, F work) {
 
 } // namespace
 
+void releaseHostTransfers() {
+    CudaContext now;
+    if (driver().getCurrent(&now.handle) != CUDA_SUCCESS || !now.handle ||
+        driver().getId(now.handle, &now.id) != CUDA_SUCCESS)
+        return;
+    std::vector<void*> blocks;
+    std::vector<HostRing*> rings;
+    {
+        std::lock_guard<std::mutex> lock(g_mutex);
+        forgetGone(now);
+        for (size_t i = g_blocks.size(); i-- > 0;)
+            if (g_blocks[i].context.id == now.id) {
+                blocks.push_back(g_blocks[i].p);
+                g_blocks.erase(g_blocks.begin() + static_cast<std::ptrdiff_t>(i));
+            }
+        for (size_t i = g_rings.size(); i-- > 0;)
+            if (g_rings[i]->context.id == now.id) {
+                rings.push_back(g_rings[i]);
+                g_rings.erase(g_rings.begin() + static_cast<std::ptrdiff_t>(i));
+                --g_ringsMade[now.id];
+            }
+    }
+    for (void* p : blocks) cudaFree(p);
+    for (HostRing* r : rings) delete r;
+}
+
+cudaError_t deviceMalloc(void** p, size_t bytes) {
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e != cudaErrorMemoryAllocation) return e;
+    cudaGetLastError();
+    releaseHostTransfers();
+    e = cudaMalloc(p, bytes);
+    if (e != cudaSuccess) cudaGetLastError();
+    return e;
+}
+
 HostTransfer::HostTransfer(size_t deviceBytes) {
     const CudaContext context = currentContext();
     contextHandle = context.handle;
     contextId = context.id;
     DeviceBlock block{ context, nullptr, deviceBytes };
     if (!takeBlock(context, deviceBytes, &block)) {
-        const cudaError_t e = cudaMalloc(&block.p, deviceBytes);
-        if (e != cudaSuccess) cudaGetLastError();
-        ck(e, "workspace");
+        ck(deviceMalloc(&block.p, deviceBytes), "workspace");
     }
     dev = block.p;
     devBytes = block.bytes;

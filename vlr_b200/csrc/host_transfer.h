@@ -14,12 +14,15 @@
 // (cudaDeviceReset); a call has its own, so calls from several threads run side by
 // side.  What is kept is bounded: two rings (calls that find
 // both in use copy through the driver), and at most eight blocks of 256 MB in
-// all; a larger block is freed when its call ends.
+// all; a larger block is freed when its call ends.  It is given back when an
+// allocation of the library fails, and with the last context object.
 // All work is on the legacy default stream, which orders it after other
 // blocking streams' work as cudaMemcpy does.
 #pragma once
 
 #include <cstddef>
+
+#include <cuda_runtime.h>
 
 struct CUctx_st;
 
@@ -53,5 +56,11 @@ private:
     HostRing* ring = nullptr;
     bool ringAsked = false;
 };
+
+// Frees the idle blocks and rings kept for the current CUDA context.
+void releaseHostTransfers();
+
+// cudaMalloc; when there is no memory left, once more without what is kept.
+cudaError_t deviceMalloc(void** p, size_t bytes);
 
 } // namespace vlrb
