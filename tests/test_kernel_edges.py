@@ -395,6 +395,47 @@ def test_kept_memory_gives_way(ray_query):
     assert build(600000) == 0
 
 
+def _device_bytes(f):
+    """Device memory that f() takes and does not give back."""
+    import torch
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    before = torch.cuda.mem_get_info()[0]
+    keep = f()
+    torch.cuda.synchronize()
+    return before - torch.cuda.mem_get_info()[0], keep
+
+
+def test_a_scene_keeps_what_rendering_reads():
+    """A grid of a million triangles: 24 B of vertices (two triangles share four of
+    them), 20 B of indices and materials, a 128 B record, 112 B of hierarchy and 52 B
+    of scratch are 336 B a triangle; a tenth for granularity."""
+    from vlr_b200 import vlr as VV
+    m = 708
+    ctx = VV.Context()
+    ctx.bindOutputBuffer(16, 16)
+    x, z = np.meshgrid(np.linspace(-1, 1, m + 1), np.linspace(-1, 1, m + 1))
+    verts = np.zeros(((m + 1) ** 2, 11), np.float32)
+    verts[:, 0], verts[:, 2], verts[:, 4], verts[:, 6] = x.ravel(), z.ravel(), 1, 1
+    i = (np.arange(m)[:, None] * (m + 1) + np.arange(m)).ravel().astype(np.uint32)
+    idx = np.stack([i, i + m + 1, i + 1, i + 1, i + m + 1, i + m + 2], axis=1).ravel()
+    mat = ctx.createSurfaceMaterial("DiffuseEmitter")
+    node = ctx.createTriangleMeshSurfaceNode("grid")
+    node.set_vertices(verts)
+    node.add_material_group(idx, mat)
+    scene = ctx.createScene()
+    scene.add_child(node)
+    cam = ctx.createCamera("Perspective")
+    cam.set_point("position", (0.0, 1.0, 2.0))
+    ctx.setScene(scene)
+    ctx.setOptions(max_path_length=2, max_paths_in_flight=256)
+    used, _ = _device_bytes(lambda: ctx.render(cam, True))
+    n = ctx.stats()["numTriangles"]
+    ctx.close()
+    assert n == 2 * m * m
+    assert used < 1.1 * 336 * n, used / n
+
+
 def _atrous(color, albedo, normal):
     """The denoiser in numpy (float64, guides rounded to halves as stored)."""
     eps = 1e-3

@@ -814,31 +814,34 @@ void Context::buildScene(cudaStream_t stream) {
 
     // ---- BVH
     if (numTris > 0) {
-        const float* dVerts = upload(f.triVerts, stream);
-        auto out = std::make_unique<DeviceBuffer>();
+        // What only the build needs (188 B a triangle) is freed once the
+        // traversal's arrays (112 B) are packed.
         const size_t n = numTris;
-        size_t off[8];
-        size_t total = 0;
-        const size_t sizes[8] = { n * 4, n * 4, n * 8, n * 24, n * sizeof(BvhNode), n * sizeof(BvhTri),
-                                  n * sizeof(TravNode), n * sizeof(BvhTri) };
-        for (int i = 0; i < 8; ++i) { off[i] = total; total += (sizes[i] + 255) & ~size_t(255); }
-        out->resize(total);
-        char* b = out->as<char>();
-        LbvhOutput lo{ reinterpret_cast<uint32_t*>(b + off[0]), reinterpret_cast<uint32_t*>(b + off[1]),
-                       reinterpret_cast<int32_t*>(b + off[2]), reinterpret_cast<float*>(b + off[3]),
-                       reinterpret_cast<BvhNode*>(b + off[4]), reinterpret_cast<BvhTri*>(b + off[5]) };
+        size_t off[7], total = 0;
+        const size_t sizes[7] = { n * 36, n * 4, n * 4, n * 8, n * 24, n * sizeof(BvhNode), n * sizeof(BvhTri) };
+        for (int i = 0; i < 7; ++i) { off[i] = total; total += (sizes[i] + 255) & ~size_t(255); }
+        DeviceBuffer built;
+        built.resize(total);
+        char* b = built.as<char>();
+        ck(cudaMemcpyAsync(b, f.triVerts.data(), n * 36, cudaMemcpyHostToDevice, stream), "triangle vertices");
+        LbvhOutput lo{ reinterpret_cast<uint32_t*>(b + off[1]), reinterpret_cast<uint32_t*>(b + off[2]),
+                       reinterpret_cast<int32_t*>(b + off[3]), reinterpret_cast<float*>(b + off[4]),
+                       reinterpret_cast<BvhNode*>(b + off[5]), reinterpret_cast<BvhTri*>(b + off[6]) };
         lbvhScratch.resize(lbvhTraversableScratchBytes(numTris));
-        bvhMaxDepth = lbvhBuildTraversable(dVerts, numTris, options.bvhTreeletRounds, lbvhScratch.ptr, &lo, nullptr,
-                                           stream);
+        bvhMaxDepth = lbvhBuildTraversable(reinterpret_cast<const float*>(b), numTris, options.bvhTreeletRounds,
+                                           lbvhScratch.ptr, &lo, nullptr, stream);
         auto flag = std::make_unique<DeviceBuffer>();
         flag->resize(256);
         ck(cudaMemsetAsync(flag->ptr, 0, 4, stream), "bvh flag");
-        TravNode* trav = reinterpret_cast<TravNode*>(b + off[6]);
-        BvhTri* travTris = reinterpret_cast<BvhTri*>(b + off[7]);
+        auto packed = std::make_unique<DeviceBuffer>();
+        packed->resize(n * (sizeof(TravNode) + sizeof(BvhTri)));
+        TravNode* trav = packed->as<TravNode>();
+        BvhTri* travTris = reinterpret_cast<BvhTri*>(trav + n);
         lbvhPackTraversal(lo, numTris, lbvhScratch.ptr, trav, travTris, flag->as<uint32_t>(), stream);
         sg.bvh = Bvh{ trav, travTris, numTris, flag->as<uint32_t>() };
         sceneBufs.push_back(std::move(flag));
-        sceneBufs.push_back(std::move(out));
+        sceneBufs.push_back(std::move(packed));
+        ck(cudaStreamSynchronize(stream), "hierarchy");
     }
 
     // ---- environment (EnvironmentEmitter with an EnvironmentTexture node)
