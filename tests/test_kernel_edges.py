@@ -436,6 +436,18 @@ def test_a_scene_keeps_what_rendering_reads():
     assert used < 1.1 * 336 * n, used / n
 
 
+def test_a_path_slot_keeps_what_path_tracing_uses():
+    """RNG 8, throughput 16, scalars 16, contribution, ray and hit 64, queues 8,
+    nine buckets 36 and a shadow ray 48: 196 B a slot."""
+    slots = 1 << 22
+    ctx, cam, keep = _render_context(64, 64, max_paths_in_flight=4096)
+    ctx.render(cam, True)
+    ctx.setOptions(max_paths_in_flight=slots)
+    used, _ = _device_bytes(lambda: ctx.render_samples(cam, True, slots // 4096))
+    ctx.close()
+    assert used < 196 * slots + (8 << 20), used / slots
+
+
 def _atrous(color, albedo, normal):
     """The denoiser in numpy (float64, guides rounded to halves as stored)."""
     eps = 1e-3

@@ -1188,9 +1188,9 @@ void Context::render(cudaStream_t stream, const Camera* cam, bool firstFrame, ui
                 if (ltCapacity < slots || ltLightSeed != lightSeed) {
                     ltLightSeed = lightSeed;
                     ltCapacity = slots;
-                    const size_t pathBytes = pathBufferBytes(slots);
+                    const size_t pathBytes = pathBufferBytes(slots, true);
                     ltMem.resize(pathBytes + ltConnectionBytes(slots));
-                    carvePathBuffers(ltMem.ptr, slots, &ltPb);
+                    carvePathBuffers(ltMem.ptr, slots, &ltPb, true);
                     ltConn = ltMem.as<char>() + pathBytes;
                     std::vector<uint64_t> seeds(slots);
                     seedPathRngs(seeds.data(), slots, lightSeed);

@@ -693,10 +693,10 @@ inline size_t a256(size_t x) { return (x + 255) & ~size_t(255); }
 
 } // namespace
 
-size_t pathBufferBytes(uint32_t P) {
+size_t pathBufferBytes(uint32_t P, bool wavelengths) {
     size_t b = 0;
     b += a256(size_t(P) * 8);                 // rng
-    b += a256(size_t(P) * 16) * 2;            // lambda, alpha
+    b += a256(size_t(P) * 16) * (wavelengths ? 2 : 1);   // lambda, alpha
     b += a256(size_t(P) * 4) * 4;             // flags, initImportance, prevDirPDF, prevType
     b += a256(size_t(P) * 16) * 4;            // contrib, rayOrg, rayDir, hit
     b += a256(size_t(P) * 4) * 2;             // active queues
@@ -707,11 +707,11 @@ size_t pathBufferBytes(uint32_t P) {
     return b;
 }
 
-void carvePathBuffers(void* base, uint32_t P, PathBuffers* pb) {
+void carvePathBuffers(void* base, uint32_t P, PathBuffers* pb, bool wavelengths) {
     char* s = static_cast<char*>(base);
     auto take = [&](size_t bytes) { char* r = s; s += a256(bytes); return r; };
     pb->rng = reinterpret_cast<uint64_t*>(take(size_t(P) * 8));
-    pb->lambda = reinterpret_cast<float4*>(take(size_t(P) * 16));
+    pb->lambda = wavelengths ? reinterpret_cast<float4*>(take(size_t(P) * 16)) : nullptr;
     pb->alpha = reinterpret_cast<float4*>(take(size_t(P) * 16));
     pb->meta = reinterpret_cast<uint4*>(s);
     pb->flags = reinterpret_cast<uint32_t*>(take(size_t(P) * 4));

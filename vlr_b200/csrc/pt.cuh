@@ -44,7 +44,7 @@ struct PathBuffers {
     uint4* meta;              // the path tracer's per-path scalars in one 16-byte record (the space of
                               // flags, initImportance, prevDirPDF and prevType): flags with prevType in
                               // bits 25-31, initImportance, prevDirPDF, and the wavelengths' offset,
-                              // from which they are computed (its lambda array is not used)
+                              // from which they are computed
     float4* alpha;
     float4* contrib;
     float* initImportance;
@@ -117,8 +117,10 @@ size_t guideBufferBytes(uint32_t numPaths, uint32_t recBounces, uint32_t sampleC
 // Carves the per-path guiding buffers (lobes, records, samples, counters).
 void carveGuideBuffers(void* base, uint32_t numPaths, uint32_t recBounces, uint32_t sampleCapacity, GuideFrame* gf);
 
-size_t pathBufferBytes(uint32_t numPaths);
-void carvePathBuffers(void* base, uint32_t numPaths, PathBuffers* pb);
+// wavelengths: with the lambda array (light tracing; the other renderers hold or
+// compute a path's wavelengths elsewhere, and lambda is null).
+size_t pathBufferBytes(uint32_t numPaths, bool wavelengths = false);
+void carvePathBuffers(void* base, uint32_t numPaths, PathBuffers* pb, bool wavelengths = false);
 
 // Seeds every path slot's PCG32 state from std::mt19937_64 in slot order, the
 // reference's per-pixel seeding (context.cpp:1176-1190) for one slot per pixel.
