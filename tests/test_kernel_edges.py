@@ -448,8 +448,9 @@ def test_a_path_slot_keeps_what_path_tracing_uses():
     assert used < 196 * slots + (8 << 20), used / slots
 
 
-def _atrous(color, albedo, normal):
-    """The denoiser in numpy (float64, guides rounded to halves as stored)."""
+def _atrous(color, albedo, normal, infinite_variance=False):
+    """The denoiser in numpy (float64, guides rounded to halves as stored).
+    infinite_variance: what FP32 makes of very bright images."""
     eps = 1e-3
     H, W = color.shape[:2]
     guided = albedo[..., :3].astype(np.float32).sum(axis=2, dtype=np.float32) > eps
@@ -465,7 +466,7 @@ def _atrous(color, albedo, normal):
             if guided[y, x]:
                 ys, xs = slice(max(y - 1, 0), y + 2), slice(max(x - 1, 0), x + 2)
                 l = L[ys, xs][guided[ys, xs]]
-                var[y, x] = max((l * l).mean() - l.mean() ** 2, 0.0)
+                var[y, x] = np.inf if infinite_variance else max((l * l).mean() - l.mean() ** 2, 0.0)
     k = [3 / 8, 1 / 4, 1 / 16]
     for step in (1, 2, 4, 8, 16):
         L = ill @ lum
@@ -488,7 +489,7 @@ def _atrous(color, albedo, normal):
                 w = w * filtered[q] * filtered[p]
                 num[p] += w[..., None] * ill[q]
                 den[p] += w
-                vs[p] += w * w * var[q]
+                vs[p] += w * w * np.where(w > 0, var[q], 0.0)
         g = filtered
         ill[g], var[g] = num[g] / den[g][:, None], vs[g] / den[g] ** 2
     out = color.astype(float).copy()
@@ -514,6 +515,46 @@ def test_denoiser_matches_numpy(size):
     off = np.abs(images[1][..., :3] - want[..., :3])
     scale = np.maximum(np.abs(want[..., :3]), np.abs(want[..., :3]).mean())
     assert (off / scale).max() < 5e-3 and (off / scale).mean() < 1e-4
+
+
+@pytest.mark.parametrize("size", [(2, 2), (6, 4), (45, 40)])
+def test_denoiser_of_a_very_bright_image(size):
+    """A floor whose illumination is about 1.3e19 everywhere: the sum of four
+    squares overflows FP32 and that of the mean does not, so the variance is
+    infinite and the luminance term drops out.  That ends in finite colours, at
+    the border too.  24 products and a quotient a pass in FP32, five passes:
+    1e-4."""
+    from vlr_b200 import vlr as VV, scenes
+    W, H = size
+
+    def render(emittance, denoise):
+        ctx = VV.Context()
+        ctx.bindOutputBuffer(W, H)
+        desc = scenes.floor_desc(W, H, light_at=(0.0, 0.0))
+        desc["camera"]["fovy"] = 0.2
+        desc["materials"]["light"] = ("DiffuseEmitter", {"emittance": ("Rec709(D65)",) + (emittance,) * 3})
+        for k, mesh in enumerate(desc["meshes"]):
+            mesh["name"] = str(k)
+        scene, cam, keep = scenes.build(ctx, desc)
+        ctx.setScene(scene)
+        ctx.setOptions(max_path_length=2, aux_buffers=True)
+        for k in range(64):
+            ctx.render(cam, k == 0, denoise=denoise and k == 63)
+        out = ctx.read_output(), ctx.read_aux()
+        ctx.close()
+        return out
+
+    lum = np.array([0.2126, 0.7152, 0.0722])
+    plain, (albedo, _) = render(1.0, False)
+    l = (plain[..., :3] / albedo[..., :3].clip(1e-3)) @ lum
+    scale = 1.3e19 / l.mean()
+    color, aux = render(scale, False)
+    l = (color[..., :3] / albedo[..., :3].clip(1e-3)) @ lum
+    assert np.isfinite(color).all() and l.min() > 0.95e19 and l.max() < 1.8e19
+    out, _ = render(scale, True)
+    want = _atrous(color, *aux, infinite_variance=True)
+    assert np.isfinite(out).all()
+    assert np.abs(out[..., :3] / want[..., :3] - 1).max() < 1e-4
 
 
 @pytest.mark.parametrize("n", [1, 127, 128, 129, 256, 257, 18944, 18945, 25000, 37888, 37889, 113664,

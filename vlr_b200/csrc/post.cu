@@ -319,7 +319,7 @@ __device__ __forceinline__ void tapPair(const WaveletCentre &c, const uint4 &g0,
                                         const float4 &i1, float h0, float h1, WaveletSums &s) {
     const float2 a0 = unpackHalf2(g0.x), b0 = unpackHalf2(g0.y), d0 = unpackHalf2(g0.z);
     const float2 a1 = unpackHalf2(g1.x), b1 = unpackHalf2(g1.y), d1 = unpackHalf2(g1.z);
-    if (a0.x < 0.0f) h0 = 0.0f;   // unguided pixels are not read
+    if (a0.x < 0.0f) h0 = 0.0f;   // unguided pixels (they hold zeros) have no weight
     if (a1.x < 0.0f) h1 = 0.0f;
     // normal term max(0, n.n')^128 by seven squarings; the albedo and
     // luminance terms in one exponential (one special-function op a tap)
@@ -347,7 +347,9 @@ __device__ __forceinline__ void tapPair(const WaveletCentre &c, const uint4 &g0,
 // filtered with the squared weights.  Bound by issue slots (25 taps of about
 // 45 instructions): taps that mirror each other share their spline weight, so
 // the 24 around the centre run as 12 pairs on packed instructions, and only
-// pixels near the border test their taps against the image.
+// pixels near the border test their taps against the image (taps outside it
+// read zeros: weight 0 must not meet an infinite variance).
+__device__ const float4 kNoTap = { 0.0f, 0.0f, 0.0f, 0.0f };
 __global__ void __launch_bounds__(256) waveletKernel(DenoiseArgs a, const float4* in, float4* out, int step) {
     const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y * blockDim.y + threadIdx.y;
     const int W = static_cast<int>(a.width), H = static_cast<int>(a.height);
@@ -376,13 +378,18 @@ __global__ void __launch_bounds__(256) waveletKernel(DenoiseArgs a, const float4
             const float h = kSpline[dx < 0 ? -dx : dx] * kSpline[dy];
             const int64_t off = dy * rowStep + dx * step;
             int64_t q0 = static_cast<int64_t>(p) + off, q1 = static_cast<int64_t>(p) - off;
+            const float4 *i0 = in + q0, *i1 = in + q1;
             float h0 = h, h1 = h;
             if (!interior) {
                 const int sx = dx * step, sy = dy * step;
-                if (x + sx < 0 || x + sx >= W || y + sy >= H) { q0 = static_cast<int64_t>(p); h0 = 0.0f; }
-                if (x - sx < 0 || x - sx >= W || y - sy < 0) { q1 = static_cast<int64_t>(p); h1 = 0.0f; }
+                if (x + sx < 0 || x + sx >= W || y + sy >= H) {
+                    q0 = static_cast<int64_t>(p); i0 = &kNoTap; h0 = 0.0f;
+                }
+                if (x - sx < 0 || x - sx >= W || y - sy < 0) {
+                    q1 = static_cast<int64_t>(p); i1 = &kNoTap; h1 = 0.0f;
+                }
             }
-            tapPair(c, a.guide[q0], a.guide[q1], in[q0], in[q1], h0, h1, s);
+            tapPair(c, a.guide[q0], a.guide[q1], *i0, *i1, h0, h1, s);
         }
     const float h = kSpline[0] * kSpline[0];
     const float sr = lo(s.r) + hi(s.r) + h * ip.x, sg = lo(s.g) + hi(s.g) + h * ip.y;
