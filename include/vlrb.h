@@ -301,6 +301,11 @@ VLRResult vlrbEvaluateSpectrum(const uint32_t packed[3], const float lambdas[4],
  * vlrbEvaluateSpectrum up to float rounding). */
 VLRResult vlrbEvaluateSpectrumTabulated(const uint32_t packed[3], const float lambdas[4], float values[4]);
 
+/* 1 when the library holds the restated spectral tables (built where the
+ * reference sources were not at hand: published definitions, not the
+ * reference's digits), 0 when it holds the reference's own. */
+uint32_t vlrbSpectralTablesRestated(void);
+
 /* The CIE 1931 colour-matching functions integrated over the 16 film strata
  * (xyz[0..15] = xbar, [16..31] = ybar, [32..47] = zbar) and the Y integral
  * (spectrum_types.cpp:634-680). */

@@ -53,6 +53,8 @@ def generate_tables(force=False):
         return
     if os.path.exists(GEN) and not _is_restated(GEN):
         return
+    print("warning: no reference sources at %s: building with the restated spectral tables "
+          "(vlrbSpectralTablesRestated() is 1)" % REFERENCE, file=sys.stderr)
     with open(RESTATED) as f:
         text = f.read()
     if os.path.exists(GEN):

@@ -50,6 +50,8 @@ extern "C" VLRResult vlrbEvaluateSpectrumTabulated(const uint32_t packed[3], con
     return VLRResult_NoError;
 }
 
+extern "C" uint32_t vlrbSpectralTablesRestated(void) { return kSpectralTablesRestated ? 1u : 0u; }
+
 extern "C" VLRResult vlrbCmfStrata(float xyz[48], float* integralCMF) {
     if (!xyz || !integralCMF) return VLRResult_InvalidArgument;
     const CmfStrata &c = hostCmfStrata();

@@ -10,6 +10,12 @@
 
 namespace vlrb {
 
+#if defined(VLRB_SPECTRAL_TABLES_RESTATED)
+const bool kSpectralTablesRestated = true;
+#else
+const bool kSpectralTablesRestated = false;
+#endif
+
 __device__ uint8_t g_mengGrid[168 * 8];
 __device__ float g_mengPoints[186 * 99];
 __device__ ColorMatrices g_colorMatrices;

@@ -7,6 +7,10 @@
 
 namespace vlrb {
 
+// Whether the tables compiled in are the restated ones instead of those
+// generated from the reference sources.
+extern const bool kSpectralTablesRestated;
+
 // Host-side views; valid for the lifetime of the process.
 MengTables hostMengTables();
 const ColorMatrices &hostColorMatrices();
