@@ -517,12 +517,12 @@ def terrain_workloads(names=("terrain_pt", "terrain_lvc_bpt"), cpu=True, paths_i
              "unit": "G path segments/s", "ms": ms,
              "stage_ms_per_spp": {k: v["ms"] / spp for k, v in stages.items() if v["ms"] > 0}}
         if renderer == V.RENDERER_PATH_TRACING:
-            dom = max(("trace", "shade", "shadow"), key=lambda k: stages[k]["ms"])
-            units = rays if dom != "shadow" else q1["shadowRays"] - q0["shadowRays"]
-            gbs = STAGE_BYTES[dom] * units / (stages[dom]["ms"] * 1e-3) / 1e9
-            r["roofline"] = {"bound": "hbm", "kernel": dom + "Kernel", "achieved": gbs, "peak": hbm_peak,
+            dom = max(STAGE_KERNELS, key=lambda k: stages[k]["ms"])
+            nbytes = stage_bytes(dom, rays, q1["shadowRays"] - q0["shadowRays"], W * H * spp)
+            gbs = nbytes / (stages[dom]["ms"] * 1e-3) / 1e9
+            r["roofline"] = {"bound": "hbm", "kernel": STAGE_KERNELS[dom], "achieved": gbs, "peak": hbm_peak,
                              "unit": "GB/s", "frac": gbs / hbm_peak, "peak_source": peak_kind,
-                             "bytes_per_unit": STAGE_BYTES[dom],
+                             "bytes_per_segment": nbytes / rays,
                              "note": "algorithmic bytes of the wavefront state; BVH node traffic excluded"}
         else:
             r["light_vertex_overflow"] = st["lightVertexOverflow"]
@@ -780,23 +780,35 @@ def batch_workload():
     return out
 
 
-# Algorithmic bytes per unit of work of each wavefront stage (SoA path state,
-# counted once per read or write; BVH traffic excluded):
-#   trace: queue index 4 + ray 32 + hit 16 + bucket append 4          = 56 B / ray
-#          (camera rays are made in the same kernel; from the second bounce on
-#          its launch also traces the shadow rays of the bounce before)
-#   shade: bucket index 4 + path scalars 16x2 + hit 16 + ray direction 16
-#          + throughput 16x2 + rng 8x2 + triangle record 120 + next ray 32
-#          + next-queue append 4 + shadow ray 48                      = 320 B / hit
-#   shadow: shadow ray 48 + contribution read-modify-write 32        = 80 B / shadow ray
-STAGE_BYTES = {"trace": 56, "shade": 320, "shadow": 80}
+# Algorithmic bytes of the path tracer's stages (SoA path state, counted once
+# per read or write; BVH traffic excluded).  The ray kernels (cameraTraceKernel at
+# the camera, then traceShadowKernel) are one stage, "trace":
+#   camera ray: rng 8x2 + path scalars 16 + throughput 16 + contribution 16
+#               + ray 32 + hit 16 + bucket append 4                  = 116 B
+#   extension ray: queue index 4 + ray 32 + hit 16 + bucket append 4 = 56 B
+#   shadow ray: shadow ray 48 + contribution read-modify-write 32    = 80 B
+# and shadeKernel's is "shade":
+#   hit: bucket index 4 + path scalars 16x2 + hit 16 + ray direction 16
+#        + throughput 16x2 + rng 8x2 + triangle record 120 + next ray 32
+#        + next-queue append 4 + shadow ray 48                       = 320 B
+STAGE_KERNELS = {"trace": "cameraTraceKernel + traceShadowKernel", "shade": "shadeKernel"}
+
+
+def stage_bytes(stage, segments, shadow_rays, paths):
+    """Algorithmic bytes of a stage over `segments` extension rays (the camera's
+    `paths` among them) and `shadow_rays`."""
+    if stage == "trace":
+        return 116 * paths + 56 * (segments - paths) + 80 * shadow_rays
+    return 320 * segments
+
+
 # DRAM bytes per path segment of each stage: dram__bytes_read.sum +
 # dram__bytes_write.sum over the 8 bounces of one launch of this workload at
 # 2^22 paths in flight (ncu, one pass), divided by that launch's segments
 # (one sixteenth of a 256-spp step); "trace" holds the camera's path-state
 # writes and the shadow rays, which have no launches of their own.  The bench's
 # own launches (2^25 paths) keep less path state in L2.
-STAGE_DRAM_BYTES_PER_SEGMENT = {"trace": 143.1, "shade": 210.7, "shadow": 0.0}
+STAGE_DRAM_BYTES_PER_SEGMENT = {"trace": 143.1, "shade": 210.7}
 
 
 def main():
@@ -919,14 +931,13 @@ def main():
     ctx.set_profiling(False)
     rays = q1["pathSegments"] - q0["pathSegments"]
     shadow = q1["shadowRays"] - q0["shadowRays"]
-    units = {"trace": rays, "shade": rays, "shadow": shadow}
     hbm_peak, peak_kind = measured_peaks()
-    dominant = max(("trace", "shade", "shadow"), key=lambda k: stages[k]["ms"])
+    dominant = max(STAGE_KERNELS, key=lambda k: stages[k]["ms"])
     st = stages[dominant]
     per_launch_ms = st["ms"] / max(st["launches"], 1)
-    bytes_per_launch = STAGE_BYTES[dominant] * units[dominant] / max(st["launches"], 1)
+    bytes_per_launch = stage_bytes(dominant, rays, shadow, 2 * W * H * SPP_PER_STEP) / max(st["launches"], 1)
     achieved = bytes_per_launch / (per_launch_ms * 1e-3) / 1e9
-    roofline = {"bound": "hbm", "kernel": dominant + "Kernel", "achieved": achieved, "peak": hbm_peak,
+    roofline = {"bound": "hbm", "kernel": STAGE_KERNELS[dominant], "achieved": achieved, "peak": hbm_peak,
                 "unit": "GB/s", "frac": achieved / hbm_peak, "traffic": None,
                 "peak_source": peak_kind,
                 "stage_ms_per_step": {k: v["ms"] / 2 for k, v in stages.items()}}

@@ -316,7 +316,11 @@ VLRResult vlrbCmfStrata(float xyz[48], float* integralCMF);
  * CUDA events on the render stream (adds a host synchronisation per render
  * call); times accumulate until reset.  Stages: 0 camera, 1 trace
  * (closest hit + material sort), 2 shade, 3 shadow rays, 4 film, 5 guiding
- * (network inference, training records, training steps).
+ * (network inference, training records, training steps).  Where kernels do
+ * two stages' work the first is charged: the path tracer's camera rays and
+ * shadow rays are in stage 1 (stages 0 and 3 stay 0), and its film pass, which
+ * also converts a finished call's image, is stage 4; light tracing's lens
+ * connections are in stage 1 but for the last vertex's, which are stage 3.
  * launchCount counts every kernel this library launched for rendering,
  * profiling on or off.
  * ---------------------------------------------------------------------- */

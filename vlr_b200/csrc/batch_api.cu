@@ -284,7 +284,7 @@ extern "C" VLRResult vlrbTraceRaysHost(const float* triVerts, uint32_t n, uint32
                                    nullptr, nullptr);
         vlrb::BvhTri* travTris = reinterpret_cast<vlrb::BvhTri*>(b + off[10]);
         vlrb::lbvhPackTraversal(lo, n, scratch, trav, travTris, flags, nullptr);
-        // the rays travel while the hierarchy's last kernels run
+        // (behind the build on the same stream; large pageable arrays are staged meanwhile)
         io.upload(b + off[7], rays, size_t(count) * 32);
         const vlrb::Bvh bvh{ trav, travTris, n, flags };
         cudaEvent_t e0, e1;

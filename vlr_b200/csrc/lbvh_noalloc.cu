@@ -7,7 +7,8 @@
 // fixed per-frame memory budget, or an embedding application whose device
 // memory is owned by its own pool (a cudaMalloc there would bypass the pool's
 // accounting, and may stall every stream of the device while it runs).  The
-// regular entry (vlrbBvhBuildHost) allocates its scratch and outputs per call.
+// regular entry (vlrbBvhBuildHost) takes its scratch and outputs from memory it
+// keeps between calls, and allocates where that does not suffice.
 //
 // Limits and rules:
 //   * at most kNoAllocMaxTriangles triangles per call (the static scratch is

@@ -157,7 +157,7 @@ __global__ void __launch_bounds__(kPersistentThreads, kPersistentMinBlocks) pers
             }
         }
         if (!end) continue;
-        // the path is done: its film sample (filmKernel's binning), then the
+        // the path is done: its film sample (the film pass's binning), then the
         // pixel's next sample or the next pixel
         alive = false;
         if (contrib.allFinite()) {
