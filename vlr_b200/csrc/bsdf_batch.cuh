@@ -197,10 +197,7 @@ __device__ __forceinline__ void shadeQueryOfRank(uint32_t rank, const BsdfBatchA
 // the sectors in L2) and outputs go back to the same slots.
 //
 // A share belongs to a group of blocks: each sorts it, and block g of the
-// group takes passes g, g + group, ...  A group of one per resident slot for
-// large batches; a batch too small to give every warp a pass that way is cut
-// into fewer, larger shares whose blocks do about one pass per warp (1021
-// queries: 56 -> 28 us).
+// group takes passes g, g + group, ...  (batchSplit).
 constexpr int kBatchThreads = 256;
 constexpr int kBatchWarps = kBatchThreads / 32;
 constexpr int kTile = 4096;
@@ -300,25 +297,32 @@ __global__ void __launch_bounds__(kBatchThreads, 3) bsdfBatchKernel(BsdfBatchArg
     }
 }
 
-// How a batch is split over the grid: see the kernel.  kWideShare queries
-// per share keep the padding of the seven last passes under a tenth.
-constexpr int64_t kWideShare = 2048, kSmallShare = 1024;
+// How a batch is split over the grid.  From kAloneShare queries per resident
+// block on, each block has a share of its own: it gives every warp about a pass
+// and more blocks sort less each.  Below, passes of a few lanes would fill the
+// GPU and fetch the same code side by side, so shares of kSmallShare queries,
+// whose passes are nearly full, are sorted by several blocks each: with nine
+// (half their warps without a pass, the others spread over more SMs) 10,000
+// queries took 26.9 us, with the five that give every warp one 29.2.  Queries of seven BSDFs, shares of their own against these: 10,000
+// 36.6 and 26.9 us, 20,000 37.1 and 31.5, 40,000 37.3 and 40.8, 100,000 49.6 and 72.3;
+// of one (Matte): 20,000 13.3 and 13.3, 100,000 13.2 and 16.7.
+constexpr int64_t kAloneShare = 72, kSmallShare = 1024, kSpreadShare = 2048;
 struct BatchSplit {
     int64_t share;
     int group, blocks;
 };
 inline BatchSplit batchSplit(int64_t n, int64_t resident) {
-    const int64_t wide = n < kWideShare ? n : kWideShare;
-    const int64_t onePass = (wide / 32 + kBatchKinds + kBatchWarps - 1) / kBatchWarps;   // blocks to give every warp a pass
-    int64_t group = resident * kWideShare / n;
-    group = group < onePass ? group : onePass;
-    if (group < 1) group = 1;
-    int64_t groups = resident / group;
-    if (groups < 1) groups = 1;
-    int64_t share = (n + groups - 1) / groups;
-    if (group > 1 && share < kSmallShare) share = kSmallShare;
+    int64_t share, group = 1;
+    if (n >= kAloneShare * resident) {
+        share = (n + resident - 1) / resident;
+    }
+    else {
+        share = n < kSmallShare ? n : kSmallShare;
+        const int64_t spread = n < kSpreadShare ? n : kSpreadShare;
+        group = (spread / 32 + kBatchKinds + kBatchWarps - 1) / kBatchWarps;
+    }
     share = (share + 7) & ~int64_t(7);
-    groups = (n + share - 1) / share;
+    const int64_t groups = (n + share - 1) / share;
     return BatchSplit{ share, static_cast<int>(group), static_cast<int>(groups * group) };
 }
 
