@@ -347,9 +347,8 @@ __device__ __forceinline__ void tapPair(const WaveletCentre &c, const uint4 &g0,
 // filtered with the squared weights.  Bound by issue slots (25 taps of about
 // 45 instructions): taps that mirror each other share their spline weight, so
 // the 24 around the centre run as 12 pairs on packed instructions, and only
-// pixels near the border test their taps against the image (taps outside it
-// read zeros: weight 0 must not meet an infinite variance).
-__device__ const float4 kNoTap = { 0.0f, 0.0f, 0.0f, 0.0f };
+// pixels near the border test their taps against the image, in code of their
+// own (taps outside it are zeros: weight 0 must not meet an infinite variance).
 __global__ void __launch_bounds__(256) waveletKernel(DenoiseArgs a, const float4* in, float4* out, int step) {
     const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y * blockDim.y + threadIdx.y;
     const int W = static_cast<int>(a.width), H = static_cast<int>(a.height);
@@ -369,28 +368,29 @@ __global__ void __launch_bounds__(256) waveletKernel(DenoiseArgs a, const float4
     const F2 zero = f2(0.0f, 0.0f);
     WaveletSums s{ zero, zero, zero, zero, zero };
     const int64_t rowStep = static_cast<int64_t>(a.stride) * step;
-    const bool interior = x >= 2 * step && y >= 2 * step && x + 2 * step < W && y + 2 * step < H;
+    auto taps = [&](auto atBorder) {
 #pragma unroll
-    for (int dy = 0; dy <= 2; ++dy)
+        for (int dy = 0; dy <= 2; ++dy)
 #pragma unroll
-        for (int dx = dy == 0 ? 1 : -2; dx <= 2; ++dx) {
-            // the tap at (dx, dy) and its mirror image
-            const float h = kSpline[dx < 0 ? -dx : dx] * kSpline[dy];
-            const int64_t off = dy * rowStep + dx * step;
-            int64_t q0 = static_cast<int64_t>(p) + off, q1 = static_cast<int64_t>(p) - off;
-            const float4 *i0 = in + q0, *i1 = in + q1;
-            float h0 = h, h1 = h;
-            if (!interior) {
-                const int sx = dx * step, sy = dy * step;
-                if (x + sx < 0 || x + sx >= W || y + sy >= H) {
-                    q0 = static_cast<int64_t>(p); i0 = &kNoTap; h0 = 0.0f;
-                }
-                if (x - sx < 0 || x - sx >= W || y - sy < 0) {
-                    q1 = static_cast<int64_t>(p); i1 = &kNoTap; h1 = 0.0f;
+            for (int dx = dy == 0 ? 1 : -2; dx <= 2; ++dx) {
+                // the tap at (dx, dy) and its mirror image
+                const float h = kSpline[dx < 0 ? -dx : dx] * kSpline[dy];
+                const int64_t off = dy * rowStep + dx * step;
+                const int64_t q0 = static_cast<int64_t>(p) + off, q1 = static_cast<int64_t>(p) - off;
+                if constexpr (!decltype(atBorder)::value) tapPair(c, a.guide[q0], a.guide[q1], in[q0], in[q1], h, h, s);
+                else {
+                    const int sx = dx * step, sy = dy * step;
+                    const bool in0 = x + sx >= 0 && x + sx < W && y + sy < H;
+                    const bool in1 = x - sx >= 0 && x - sx < W && y - sy >= 0;
+                    const float4 none = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                    tapPair(c, in0 ? a.guide[q0] : gp, in1 ? a.guide[q1] : gp, in0 ? in[q0] : none,
+                            in1 ? in[q1] : none, in0 ? h : 0.0f, in1 ? h : 0.0f, s);
                 }
             }
-            tapPair(c, a.guide[q0], a.guide[q1], *i0, *i1, h0, h1, s);
-        }
+    };
+    const bool interior = x >= 2 * step && y >= 2 * step && x + 2 * step < W && y + 2 * step < H;
+    if (__all_sync(__activemask(), interior)) taps(std::false_type{});
+    else taps(std::true_type{});   // the whole warp, so that none runs both
     const float h = kSpline[0] * kSpline[0];
     const float sr = lo(s.r) + hi(s.r) + h * ip.x, sg = lo(s.g) + hi(s.g) + h * ip.y;
     const float sb = lo(s.b) + hi(s.b) + h * ip.z, wsum = lo(s.w) + hi(s.w) + h;
