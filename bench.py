@@ -339,10 +339,10 @@ def time_to_rmse():
 # ---- the other scope-table workloads, reported beside the headline line
 BATCH_BYTES_PER_QUERY = 116     # in: wo 12, material 4, roughness 8, ior 4, albedo 12, metallic 4, u 12,
                                 # wavelength u 8; out: value 16, pdf 4, wi 12, eval value 16, eval pdf 4
-# ncu, one launch of the 2^20-query batch (--set full): DRAM bytes read +
+# ncu, one launch of the 2^20-query batch: DRAM bytes read +
 # written, FMA-pipe and issue-active fractions; the kernel is issue/latency
 # bound inside the GGX BSDFs, so these stand beside its HBM fraction.
-BATCH_NCU = {"dram_bytes": 177.8e6 + 93.7e6, "fma_pipe": 0.243, "issue": 0.480}
+BATCH_NCU = {"dram_bytes": 139.3e6 + 52.9e6, "fma_pipe": 0.223, "issue": 0.494}
 
 
 def bsdf_batch_workload(hbm_peak):
@@ -808,7 +808,7 @@ def stage_bytes(stage, segments, shadow_rays, paths):
 # (one sixteenth of a 256-spp step); "trace" holds the camera's path-state
 # writes and the shadow rays, which have no launches of their own.  The bench's
 # own launches (2^25 paths) keep less path state in L2.
-STAGE_DRAM_BYTES_PER_SEGMENT = {"trace": 143.1, "shade": 210.7}
+STAGE_DRAM_BYTES_PER_SEGMENT = {"trace": 141.8, "shade": 208.5}
 
 
 def main():
