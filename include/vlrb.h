@@ -234,6 +234,13 @@ VLRResult vlrbContextGetOutputDevicePointer(VLRContext context, void** devicePtr
  *                   ~i leaf i in sorted order)
  *   nodeBoxes[6(n-1)] box (min xyz, max xyz) of each internal node
  * buildMs (may be NULL) receives the GPU build time.
+ *
+ * The calls here and below that take host arrays (hierarchies, ray queries,
+ * the guiding network) keep device memory (at most 256 MB) and pinned staging
+ * slots (at most 16 MB) between calls, per CUDA context; it is released when
+ * an allocation of the library fails and when the last VLRContext is
+ * destroyed, and forgotten after cudaDeviceReset.  Calls from several threads
+ * run side by side.  Pinned arrays are copied directly, pageable ones staged.
  * ---------------------------------------------------------------------- */
 VLRResult vlrbBvhBuildHost(const float* triVerts, uint32_t n, uint32_t* sortedCodes, uint32_t* sortedPrims,
                            int32_t* children, float* nodeBoxes, float* buildMs);
