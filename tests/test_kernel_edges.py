@@ -416,7 +416,11 @@ def test_kept_memory_gives_way(ray_query):
     ctx.close()
     del keep
     assert free() > held + 140 * MB
+    before = free()
+    assert build(1200000) == 0                   # about 300 MB: above what is kept
+    assert free() > before - 8 * MB
     assert build(600000) == 0
+    assert np.array_equal(_trace(*ray_query[:2]).view(np.uint32), ray_query[2].view(np.uint32))
 
 
 @pytest.mark.parametrize("size", [(1, 1), (7, 3), (33, 17), (129, 5)])

@@ -85,7 +85,7 @@ struct AuxArgs {
 // is atomic, and the linear images come from the sums just formed instead of
 // a second pass over 128 B a pixel.  kAdd: to what the buffers hold, else in its
 // place; its lines are read ahead of the stores (1920 x 1080 guides added: 0.42 ->
-// 0.36 ms, in one step after the other the compiler keeps load and store apart).
+// 0.36 ms; the compiler has to keep loads behind stores that it cannot tell apart).
 // The white point, the same for every pixel, is tabulated in shared memory;
 // upsampling it took six gathers a wavelength (denoised 1080p frame 1.67 -> 1.61
 // ms).
