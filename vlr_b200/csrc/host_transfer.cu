@@ -9,6 +9,7 @@
 #include <exception>
 #include <map>
 #include <mutex>
+#include <new>
 #include <stdexcept>
 #include <string>
 #include <system_error>
@@ -101,50 +102,65 @@ const Driver &driver() {
     return d;
 }
 
+// The current context; false where there is none, or only the handle of one
+// that is gone.
+bool askContext(CudaContext* c) {
+    return driver().getCurrent(&c->handle) == CUDA_SUCCESS && c->handle &&
+           driver().getId(c->handle, &c->id) == CUDA_SUCCESS;
+}
+
 CudaContext currentContext() {
-    ck(cudaFree(nullptr), "context");   // makes the device's primary context if none is current
     CudaContext c;
-    if (driver().getCurrent(&c.handle) != CUDA_SUCCESS || !c.handle ||
-        driver().getId(c.handle, &c.id) != CUDA_SUCCESS)
-        throw std::runtime_error("host transfer: no CUDA context");
+    if (askContext(&c)) return c;
+    ck(cudaFree(nullptr), "context");   // makes the device's primary context
+    if (!askContext(&c)) throw std::runtime_error("host transfer: no CUDA context");
     return c;
 }
 
-// Idle ones.
-std::mutex g_mutex;
-std::vector<DeviceBlock> g_blocks;
-std::vector<HostRing*> g_rings;
-std::map<unsigned long long, int> g_ringsMade;   // per context, idle or borrowed
+// What is idle.  Never destroyed: the last context object may go after this
+// library's static objects.
+struct Kept {
+    std::mutex mutex;
+    std::vector<DeviceBlock> blocks;
+    std::vector<HostRing*> rings;
+    std::map<unsigned long long, int> ringsMade;   // per context, idle or borrowed
+};
+Kept &kept() {
+    static Kept* const k = new Kept;
+    return *k;
+}
 
 // Forgets what was kept of a context that is gone: its handle is `now`'s, its
 // id is not.  (With the mutex held.)
 void forgetGone(const CudaContext &now) {
+    Kept &k = kept();
     auto gone = [&](const CudaContext &c) { return c.handle == now.handle && c.id != now.id; };
-    g_blocks.erase(std::remove_if(g_blocks.begin(), g_blocks.end(), [&](const DeviceBlock &b) { return gone(b.context); }),
-                   g_blocks.end());
-    for (HostRing* &r : g_rings)
+    k.blocks.erase(std::remove_if(k.blocks.begin(), k.blocks.end(), [&](const DeviceBlock &b) { return gone(b.context); }),
+                   k.blocks.end());
+    for (HostRing* &r : k.rings)
         if (gone(r->context)) {
-            g_ringsMade.erase(r->context.id);
+            k.ringsMade.erase(r->context.id);
             r->pinned = nullptr;
             for (cudaEvent_t &e : r->done) e = nullptr;
             delete r;
             r = nullptr;
         }
-    g_rings.erase(std::remove(g_rings.begin(), g_rings.end(), nullptr), g_rings.end());
+    k.rings.erase(std::remove(k.rings.begin(), k.rings.end(), nullptr), k.rings.end());
 }
 
 // The smallest idle block of at least `bytes`.
 bool takeBlock(const CudaContext &context, size_t bytes, DeviceBlock* out) {
-    std::lock_guard<std::mutex> lock(g_mutex);
+    Kept &k = kept();
+    std::lock_guard<std::mutex> lock(k.mutex);
     forgetGone(context);
-    size_t best = g_blocks.size();
-    for (size_t i = 0; i < g_blocks.size(); ++i)
-        if (g_blocks[i].context.id == context.id && g_blocks[i].bytes >= bytes &&
-            (best == g_blocks.size() || g_blocks[i].bytes < g_blocks[best].bytes))
+    size_t best = k.blocks.size();
+    for (size_t i = 0; i < k.blocks.size(); ++i)
+        if (k.blocks[i].context.id == context.id && k.blocks[i].bytes >= bytes &&
+            (best == k.blocks.size() || k.blocks[i].bytes < k.blocks[best].bytes))
             best = i;
-    if (best == g_blocks.size()) return false;
-    *out = g_blocks[best];
-    g_blocks.erase(g_blocks.begin() + static_cast<std::ptrdiff_t>(best));
+    if (best == k.blocks.size()) return false;
+    *out = k.blocks[best];
+    k.blocks.erase(k.blocks.begin() + static_cast<std::ptrdiff_t>(best));
     return true;
 }
 
@@ -152,23 +168,28 @@ bool takeBlock(const CudaContext &context, size_t bytes, DeviceBlock* out) {
 void keepBlock(const DeviceBlock &block) {
     std::vector<void*> dropped;
     {
-        std::lock_guard<std::mutex> lock(g_mutex);
-        size_t count = 0, bytes = 0;
-        for (const DeviceBlock &k : g_blocks)
-            if (k.context.id == block.context.id) { ++count; bytes += k.bytes; }
-        while (block.bytes <= kKeptBytes && (count + 1 > kKeptBlocks || bytes + block.bytes > kKeptBytes)) {
-            auto least = g_blocks.end();
-            for (auto i = g_blocks.begin(); i != g_blocks.end(); ++i)
+        Kept &k = kept();
+        std::lock_guard<std::mutex> lock(k.mutex);
+        size_t count = 0, bytes = 0, stayCount = 0, stayBytes = 0;
+        for (const DeviceBlock &b : k.blocks)
+            if (b.context.id == block.context.id) {
+                ++count;
+                bytes += b.bytes;
+                if (b.bytes >= block.bytes) { ++stayCount; stayBytes += b.bytes; }
+            }
+        const bool fits = stayCount + 1 <= kKeptBlocks && stayBytes + block.bytes <= kKeptBytes;
+        while (fits && (count + 1 > kKeptBlocks || bytes + block.bytes > kKeptBytes)) {
+            auto least = k.blocks.end();
+            for (auto i = k.blocks.begin(); i != k.blocks.end(); ++i)
                 if (i->context.id == block.context.id && i->bytes < block.bytes &&
-                    (least == g_blocks.end() || i->bytes < least->bytes))
+                    (least == k.blocks.end() || i->bytes < least->bytes))
                     least = i;
-            if (least == g_blocks.end()) break;
             --count;
             bytes -= least->bytes;
             dropped.push_back(least->p);
-            g_blocks.erase(least);
+            k.blocks.erase(least);
         }
-        if (count + 1 <= kKeptBlocks && bytes + block.bytes <= kKeptBytes) g_blocks.push_back(block);
+        if (fits) k.blocks.push_back(block);
         else dropped.push_back(block.p);
     }
     for (void* p : dropped) cudaFree(p);
@@ -176,16 +197,17 @@ void keepBlock(const DeviceBlock &block) {
 
 // An idle ring, a new one, or null: the caller then copies through the driver.
 HostRing* takeRing(const CudaContext &context) {
+    Kept &k = kept();
     {
-        std::lock_guard<std::mutex> lock(g_mutex);
-        for (size_t i = 0; i < g_rings.size(); ++i)
-            if (g_rings[i]->context.id == context.id) {
-                HostRing* r = g_rings[i];
-                g_rings.erase(g_rings.begin() + static_cast<std::ptrdiff_t>(i));
+        std::lock_guard<std::mutex> lock(k.mutex);
+        for (size_t i = 0; i < k.rings.size(); ++i)
+            if (k.rings[i]->context.id == context.id) {
+                HostRing* r = k.rings[i];
+                k.rings.erase(k.rings.begin() + static_cast<std::ptrdiff_t>(i));
                 return r;
             }
-        if (g_ringsMade[context.id] >= kRings) return nullptr;
-        ++g_ringsMade[context.id];
+        if (k.ringsMade[context.id] >= kRings) return nullptr;
+        ++k.ringsMade[context.id];
     }
     HostRing* r = new HostRing;
     r->context = context;
@@ -195,15 +217,16 @@ HostRing* takeRing(const CudaContext &context) {
     if (ok) return r;
     cudaGetLastError();
     delete r;
-    std::lock_guard<std::mutex> lock(g_mutex);
-    --g_ringsMade[context.id];
+    std::lock_guard<std::mutex> lock(k.mutex);
+    --k.ringsMade[context.id];
     return nullptr;
 }
 
 void returnRing(HostRing* r, bool idle) {
-    std::lock_guard<std::mutex> lock(g_mutex);
-    if (idle) { g_rings.push_back(r); return; }
-    --g_ringsMade[r->context.id];
+    Kept &k = kept();
+    std::lock_guard<std::mutex> lock(k.mutex);
+    if (idle) { k.rings.push_back(r); return; }
+    --k.ringsMade[r->context.id];
     delete r;
 }
 
@@ -249,27 +272,35 @@ void runWorkers(const CudaContext &context, size_t bytes, F work) {
 
 } // namespace
 
-void releaseHostTransfers() {
-    CudaContext now;
-    if (driver().getCurrent(&now.handle) != CUDA_SUCCESS || !now.handle ||
-        driver().getId(now.handle, &now.id) != CUDA_SUCCESS)
-        return;
+void releaseHostTransfers() noexcept {
     std::vector<void*> blocks;
     std::vector<HostRing*> rings;
-    {
-        std::lock_guard<std::mutex> lock(g_mutex);
+    try {
+        Kept &k = kept();
+        {
+            std::lock_guard<std::mutex> lock(k.mutex);
+            if (k.blocks.empty() && k.rings.empty()) return;
+        }
+        CudaContext now;
+        if (!askContext(&now)) return;
+        std::lock_guard<std::mutex> lock(k.mutex);
         forgetGone(now);
-        for (size_t i = g_blocks.size(); i-- > 0;)
-            if (g_blocks[i].context.id == now.id) {
-                blocks.push_back(g_blocks[i].p);
-                g_blocks.erase(g_blocks.begin() + static_cast<std::ptrdiff_t>(i));
+        blocks.reserve(k.blocks.size());
+        rings.reserve(k.rings.size());
+        for (size_t i = k.blocks.size(); i-- > 0;)
+            if (k.blocks[i].context.id == now.id) {
+                blocks.push_back(k.blocks[i].p);
+                k.blocks.erase(k.blocks.begin() + static_cast<std::ptrdiff_t>(i));
             }
-        for (size_t i = g_rings.size(); i-- > 0;)
-            if (g_rings[i]->context.id == now.id) {
-                rings.push_back(g_rings[i]);
-                g_rings.erase(g_rings.begin() + static_cast<std::ptrdiff_t>(i));
-                --g_ringsMade[now.id];
+        for (size_t i = k.rings.size(); i-- > 0;)
+            if (k.rings[i]->context.id == now.id) {
+                rings.push_back(k.rings[i]);
+                k.rings.erase(k.rings.begin() + static_cast<std::ptrdiff_t>(i));
+                --k.ringsMade[now.id];
             }
+    }
+    catch (...) {
+        return;   // no driver left to ask (the process ends), or no memory: nothing is released
     }
     for (void* p : blocks) cudaFree(p);
     for (HostRing* r : rings) delete r;
@@ -300,9 +331,14 @@ HostTransfer::HostTransfer(size_t deviceBytes) {
 HostTransfer::~HostTransfer() {
     // nothing of this call may still use what another takes
     const bool idle = cudaStreamSynchronize(nullptr) == cudaSuccess;
-    if (ring) returnRing(ring, idle);
-    if (idle) keepBlock(DeviceBlock{ { contextHandle, contextId }, dev, devBytes });
-    else cudaFree(dev);
+    try {
+        if (ring) returnRing(ring, idle);
+        if (idle) keepBlock(DeviceBlock{ { contextHandle, contextId }, dev, devBytes });
+        else cudaFree(dev);
+    }
+    catch (const std::bad_alloc &) {
+        // no host memory to note what is kept: it is not
+    }
 }
 
 void* HostTransfer::device() const { return dev; }

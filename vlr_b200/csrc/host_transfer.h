@@ -59,8 +59,9 @@ private:
     bool ringAsked = false;
 };
 
-// Frees the idle blocks and rings kept for the current CUDA context.
-void releaseHostTransfers();
+// Frees the idle blocks and rings kept for the current CUDA context (called from
+// destructors too, at the process's end among them).
+void releaseHostTransfers() noexcept;
 
 // cudaMalloc; when there is no memory left, once more without what is kept.
 cudaError_t deviceMalloc(void** p, size_t bytes);
